@@ -746,11 +746,11 @@ def build_matrix(basis, op_list, dtype):
         fl = D.to_host(flags)
         moved = [off_idx[k] for k in range(len(off_idx)) if (fl[k] & 1) and not (fl[k] & 2)]
         dropped = [off_idx[k] for k in range(len(off_idx)) if not (fl[k] & 1)]
-        if not moved and not dropped:
-            break
         for i in moved:
             is_diag[i] = True
         off_idx = [i for i in off_idx if i not in moved and i not in dropped]
+        if not moved:
+            break           # terms without elements added nothing to the counts
     diag_idx = [i for i, d in enumerate(is_diag) if d]
     diag = None
     if diag_idx and Ns:
