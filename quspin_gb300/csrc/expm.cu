@@ -341,7 +341,8 @@ extern "C" int qs_taylor_term_rows(int64_t n, int64_t nnz, const void *indptr, i
                  ctl, G, U, co, co && ((group >> 17) & 1), rownorm, st};
         a.occ = group > 0 ? (group >> 18) & 3 : 0;
         a.nnz = nnz;
-        a.staged = group > 0 ? (group >> 20) & 7 : 0;
+        // several vectors without a given shape: the vectors across the lanes
+        a.staged = group > 0 ? (group >> 20) & 7 : (nvec > 1 ? 1 : 0);
         if (a.staged) return a.nvec == 1 ? st_taylor_term(a) : vl_taylor_term(a, false);
         return lp_taylor_term(a, false);
     }
@@ -668,7 +669,7 @@ extern "C" int qs_taylor_multi_term_rows(int64_t n, const void *indptr, const in
         LpTerm a{n, indptr, 0, indices, data, dtype, Bin, Bout, btype, Fp, nvec, cdbl{0.0, 0.0}, m, sec_off, cf, j, tol,
                  ctl, G, U, co, co && ((group >> 17) & 1), rownorm, st};
         a.occ = group > 0 ? (group >> 18) & 3 : 0;
-        a.staged = group > 0 ? (group >> 20) & 7 : 0;
+        a.staged = group > 0 ? (group >> 20) & 7 : (nvec > 1 ? 1 : 0);
         if (a.staged && nvec > 1) return vl_taylor_term(a, true);
         return lp_taylor_term(a, true);
     }

@@ -37,7 +37,7 @@
 #include <type_traits>
 #include "expm_ctl.cuh"
 #include "pairf.cuh"
-#include "lp_modes.cuh"
+#include "lp_lanes.cuh"
 
 namespace {
 
@@ -424,25 +424,25 @@ __global__ void __launch_bounds__(256) taylor_lp_load_kernel(int64_t n, int64_t 
 {
     constexpr int NS = MULTI ? QS_MAX_SECTORS : 1;
     __shared__ int64_t s_off[NS + 1];
-    __shared__ double s_sc[NS];
+    __shared__ int s_bexp[NS];
     int nsec = 1;
     if constexpr (MULTI) {
         const MultiCtl *ctl = reinterpret_cast<const MultiCtl *>(ctlp);
         nsec = ctl->nsec;
         for (int b = threadIdx.x; b <= nsec; b += blockDim.x) s_off[b] = sec_off[b];
-        for (int b = threadIdx.x; b < nsec; b += blockDim.x) s_sc[b] = pow2(-ctl->bexp[b]);
+        for (int b = threadIdx.x; b < nsec; b += blockDim.x) s_bexp[b] = ctl->bexp[b];
     } else {
-        if (threadIdx.x == 0) s_sc[0] = pow2(-reinterpret_cast<const ExpmCtl *>(ctlp)->bexp);
+        if (threadIdx.x == 0) s_bexp[0] = reinterpret_cast<const ExpmCtl *>(ctlp)->bexp;
     }
     __syncthreads();
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         int b = 0;
         if constexpr (MULTI) b = sector_of(s_off, nsec, r);
-        const double sc = s_sc[b];
+        const int bexp = s_bexp[b];
         for (int64_t c = 0; c < nvec; c++) {
             const int64_t e = r * nvec + c;
             const cdbl f = F[e];
-            M::st(B0 + e, typename M::BE{M::from_d(f.x * sc), M::from_d(f.y * sc)});
+            M::st(B0 + e, typename M::BE{scaled_from_double<M>(f.x, bexp), scaled_from_double<M>(f.y, bexp)});
         }
     }
 }
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(256) taylor_lp_load_kernel(int64_t n, int64_t 
 __global__ void split_pairs_kernel(int64_t count, const double *__restrict__ src, float2 *__restrict__ dst)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        const pf v = pf_from_double(src[i]);
+        const pf v = pair_rn_scaled(src[i], 0);
         dst[i] = make_float2(v.h, v.l);
     }
 }

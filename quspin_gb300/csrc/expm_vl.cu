@@ -12,29 +12,31 @@
 // instructions, each of which touches 32 different cache lines, one per lane.
 // Measured with ncu on the L=22 Ising sectors (8 vectors), the L1TEX data
 // pipe is then the busy unit (73% of its wavefronts, DRAM at 13%).  Here a
-// group of 8 lanes owns a row and lane v owns vector c0 + v: one warp load
-// gathers the whole 128-byte rows of B for four nonzeros (one per group), so
-// a nonzero costs one wavefront instead of eight; each lane keeps one
-// accumulator pair instead of eight, and a row's sums need no cross-lane
-// merge.  The products, the epilogue and the F update use the arithmetic of
-// csrc/expm_lp.cu; one lane sums a row's nonzeros in order, and the row sums
-// of moduli add the vectors in a butterfly, so results agree with that kernel
-// to float-pair rounding.
+// group of 8 lanes (2 or 4 for as few vectors) owns a row and lane v owns
+// vector c0 + v: one warp load gathers the whole 128-byte rows of B for four
+// nonzeros (one per group), so a nonzero costs one wavefront instead of eight;
+// each lane keeps one accumulator pair instead of eight, and a row's sums need
+// no cross-lane merge.  The products, the epilogue and the F update use the
+// arithmetic of csrc/expm_lp.cu; one lane sums a row's nonzeros in order, and
+// the row sums of moduli add the vectors in a butterfly, so results agree with
+// that kernel to float-pair rounding.  The row loop is vl_row_sum
+// (lp_lanes.cuh); with every lane loading each nonzero's column itself, two in
+// flight, the L=16 sector stack (65536 rows, 17 nonzeros, 8 vectors) took
+// 44.6 us a launch on average over an evolution, 40 us now.
 #include "qs_common.cuh"
 #include <type_traits>
 #include "expm_ctl.cuh"
 #include "pairf.cuh"
-#include "lp_modes.cuh"
+#include "lp_lanes.cuh"
 
 namespace {
 
-constexpr int VL = 8;    // lanes per row group = vectors per sweep of a row
-
-template <class M, class DV, class IT, int U, bool MULTI, bool CODED>
+// VL: lanes per row group = vectors per sweep of a row; WPL: as vl_row_sum
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
 __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices,
                                         const DV *__restrict__ data, const typename M::BE *__restrict__ Bin,
                                         typename M::BE *__restrict__ Bout, cdbl *__restrict__ F, int64_t nvec,
-                                        cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,
+                                        int VL, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,
                                         const cdbl *__restrict__ coeff, int j, double tol, void *ctlp)
 {
     using S = typename M::S;
@@ -78,6 +80,7 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
     }
     if (threadIdx.x == 32) s_cf[0] = M::from_d(coeff[j].x);
     if (threadIdx.x == 33) s_cf[1] = M::from_d(coeff[j].y);
+    constexpr bool CODED = VMODE != 0;
     __shared__ DV s_tab[CODED ? QS_CODE_TABLE : 1];
     const uint8_t *codes = nullptr;
     if constexpr (CODED) {
@@ -86,9 +89,8 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
     }
     __syncthreads();
 
-    const int v = threadIdx.x & (VL - 1);
-    const int grp = (threadIdx.x & 31) / VL;
-    constexpr int RPW = 32 / VL;             // rows per warp and sweep
+    // 32 / VL rows per warp and sweep
+    const int RPW = 32 / VL, grp = (threadIdx.x & 31) / VL, lane0 = grp * VL, v = (threadIdx.x & 31) - lane0;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const S cf_re = s_cf[0], cf_im = s_cf[1];
@@ -97,33 +99,17 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
         const int64_t r = rb + grp;
         int sec = 0;
         if constexpr (MULTI) sec = r < n ? sector_of(s_off, nsec, r) : 0;
-        const bool valid = r < n && !s_done[sec];
+        const bool valid = r < n && grp < RPW && !s_done[sec];
         const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
         const int bexp = s_bexp[sec];
         const S cm_re = s_cm[2 * sec], cm_im = s_cm[2 * sec + 1];
         pf rbp{0.f, 0.f}, rfp{0.f, 0.f};
         for (int64_t c0 = 0; c0 < nvec; c0 += VL) {
-            const int64_t c = c0 + v;
-            const bool act = valid && c < nvec;
+            const int64_t c = c0 + v < nvec ? c0 + v : nvec - 1;
+            const bool act = valid && c0 + v < nvec;
             S ar = M::zero(), ai = M::zero();
-            for (IT k = k0; k < k1; k += (IT)U) {
-                int32_t col[U];
-                DV d[U];
-                BE bv[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const bool in = k + (IT)u < k1;
-                    col[u] = in ? __ldcs(indices + k + u) : 0;
-                    if constexpr (CODED) d[u] = in ? s_tab[__ldcs(codes + k + u)] : vzero<DV>();
-                    else d[u] = in ? ldv(data + k + u) : vzero<DV>();
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++)
-                    bv[u] = (act && k + (IT)u < k1) ? M::ldB(Bin + (int64_t)col[u] * nvec + c) : BE{M::zero(), M::zero()};
-#pragma unroll
-                for (int u = 0; u < U; u++)
-                    if (k + (IT)u < k1) vmul_acc<M>(ar, ai, d[u], bv[u]);
-            }
+            vl_row_sum<M, DV, true, IT, VMODE, WPL>(indices, data, codes, s_tab, Bin + c,
+                                                    (uint32_t)(nvec * sizeof(BE)), v, lane0, grp < RPW, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
                 const BE bo = M::ldB(Bin + e);
@@ -145,11 +131,14 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
                 rfp = pf_add(rfp, pf_sqrt(pf_add(pf_mul(fr, fr), pf_mul(fi, fi))));
             }
         }
-        // the row's sums of moduli over its vectors: the group's eight lanes
-#pragma unroll
+        // the row's sums of moduli over its vectors: a tree over the group's
+        // lanes, complete in lane 0
         for (int o = 1; o < VL; o <<= 1) {
-            rbp = pf_add(rbp, shfl_xor_pair(rbp, o));
-            rfp = pf_add(rfp, shfl_xor_pair(rfp, o));
+            const pf tb = shfl_pair(rbp, (threadIdx.x & 31) + o), tf = shfl_pair(rfp, (threadIdx.x & 31) + o);
+            if (v + o < VL) {
+                rbp = pf_add(rbp, tb);
+                rfp = pf_add(rfp, tf);
+            }
         }
         if (valid && v == 0) {
             const double rbn = pf_to_double_scaled(rbp, 0), rfn = pf_to_double_scaled(rfp, 0);
@@ -215,75 +204,74 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
 #define VL_PARAMS                                                                                             \
     int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices, const DV *__restrict__ data, \
         const typename M::BE *__restrict__ Bin, typename M::BE *__restrict__ Bout, cdbl *__restrict__ F,         \
-        int64_t nvec, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,              \
+        int64_t nvec, int VL, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,              \
         const cdbl *__restrict__ coeff, int j, double tol, void *ctlp
-#define VL_ARGS n, indptr, indices, data, Bin, Bout, F, nvec, mu0, mus, sec_off, coeff, j, tol, ctlp
+#define VL_ARGS n, indptr, indices, data, Bin, Bout, F, nvec, VL, mu0, mus, sec_off, coeff, j, tol, ctlp
 
-template <class M, class DV, class IT, int U, bool MULTI, bool CODED>
-__global__ void __launch_bounds__(256, 4) taylor_vl_kernel(VL_PARAMS)
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
+__global__ void __launch_bounds__(256, 3) taylor_vl_kernel(VL_PARAMS)
 {
-    vl_body<M, DV, IT, U, MULTI, CODED>(VL_ARGS);
-}
-template <class M, class DV, class IT, int U, bool MULTI, bool CODED>
-__global__ void __launch_bounds__(256, 5) taylor_vl_kernel_occ5(VL_PARAMS)
-{
-    vl_body<M, DV, IT, U, MULTI, CODED>(VL_ARGS);
+    vl_body<M, DV, IT, WPL, MULTI, VMODE>(VL_ARGS);
 }
 
-template <class M, class DV, class IT, int U, bool MULTI, bool CODED, bool OCC5>
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
 int vl_go(const LpTerm &a)
 {
     using BE = typename M::BE;
     static int resident = 0;
-    auto k = OCC5 ? taylor_vl_kernel_occ5<M, DV, IT, U, MULTI, CODED> : taylor_vl_kernel<M, DV, IT, U, MULTI, CODED>;
-    const int64_t need = (a.n + 31) / 32;          // 32 rows per block and sweep
-    const int blocks = qs_persistent_grid(k, 256, need, resident);
+    auto k = taylor_vl_kernel<M, DV, IT, WPL, MULTI, VMODE>;
+    const int VL = vl_lanes(a.nvec);
+    const int64_t rows = 8 * (32 / VL);       // per block and sweep
+    const int blocks = qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident);
     k<<<blocks, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, (const BE *)a.Bin,
-                                (BE *)a.Bout, a.F, a.nvec, a.mu0, a.mus, a.sec_off, a.coeff, a.j, a.tol, a.ctl);
+                                (BE *)a.Bout, a.F, a.nvec, VL, a.mu0, a.mus, a.sec_off, a.coeff, a.j, a.tol, a.ctl);
     QS_CHECK(cudaGetLastError());
     return QS_OK;
 }
 
-// a.staged: 1 four nonzeros in flight per lane, 4 blocks per SM; 2 two in
-// flight, 4 blocks; 3 two in flight, registers capped for 5 blocks per SM
-template <class M, class DV, class IT, bool MULTI, bool CODED>
+template <class M, class DV, class IT, bool MULTI, int VMODE>
 int vl_shape(const LpTerm &a)
 {
-    switch (a.staged) {
-    case 1: return vl_go<M, DV, IT, 4, MULTI, CODED, false>(a);
-    case 2: return vl_go<M, DV, IT, 2, MULTI, CODED, false>(a);
-    case 3: return vl_go<M, DV, IT, 2, MULTI, CODED, true>(a);
-    default: return QS_ERR_ARG;
-    }
+    if (a.nvec <= 3) return vl_go<M, DV, IT, 2, MULTI, VMODE>(a);
+    return vl_go<M, DV, IT, 1, MULTI, VMODE>(a);
 }
 
-template <class M, class DV, bool MULTI, bool CODED = false>
+template <class M, class DV, bool MULTI, int VMODE = 0>
 int vl_idx(const LpTerm &a)
 {
-    if constexpr (CODED) {
+    if constexpr (VMODE != 0) {
         if (a.idx64) return QS_ERR_ARG;
-        return vl_shape<M, DV, int32_t, MULTI, true>(a);
+        return vl_shape<M, DV, int32_t, MULTI, VMODE>(a);
     } else {
-        if (a.idx64) return vl_shape<M, DV, int64_t, MULTI, false>(a);
-        return vl_shape<M, DV, int32_t, MULTI, false>(a);
+        if constexpr (!MULTI) {
+            if (a.idx64) return vl_shape<M, DV, int64_t, MULTI, 0>(a);
+        }
+        return vl_shape<M, DV, int32_t, MULTI, 0>(a);
     }
 }
 
 }  // namespace
 
 // The float forms' term for nvec > 1 vectors with the vectors across the
-// lanes (a.staged = 1..3: see vl_shape); one matrix or a stack of sectors.
+// lanes; one matrix or a stack of sectors.  a.staged = 1..3 (one kernel:
+// registers for three blocks per SM; the epilogue spills at four, measured 2 to
+// 10% slower, and more at five, 15%).
 int vl_taylor_term(const LpTerm &a, bool multi)
 {
-    if (a.nvec < 2 || a.staged < 1 || a.staged > 3) return QS_ERR_ARG;
+    if (a.nvec < 2 || a.nvec >= (1 << 27) || a.staged < 1 || a.staged > 3) return QS_ERR_ARG;
     if (multi && a.idx64) return QS_ERR_ARG;
     if (a.btype == QS_CPF) {
-        if (a.dtype == QS_PF) return multi ? vl_idx<ModePF, pf, true>(a) : vl_idx<ModePF, pf, false>(a);
-        if (a.dtype == QS_CPF) return multi ? vl_idx<ModePF, cpf, true>(a) : vl_idx<ModePF, cpf, false>(a);
-        if (a.dtype == QS_PF8) return multi ? vl_idx<ModePF, pf, true, true>(a) : vl_idx<ModePF, pf, false, true>(a);
-        if (a.dtype == QS_CPF8)
-            return multi ? vl_idx<ModePF, cpf, true, true>(a) : vl_idx<ModePF, cpf, false, true>(a);
-    } else if (a.btype == QS_C64) {
+        switch (a.dtype) {
+        case QS_PF: return multi ? vl_idx<ModePF, pf, true>(a) : vl_idx<ModePF, pf, false>(a);
+        case QS_CPF: return multi ? vl_idx<ModePF, cpf, true>(a) : vl_idx<ModePF, cpf, false>(a);
+        case QS_PF8: return multi ? vl_idx<ModePF, pf, true, 1>(a) : vl_idx<ModePF, pf, false, 1>(a);
+        case QS_CPF8: return multi ? vl_idx<ModePF, cpf, true, 1>(a) : vl_idx<ModePF, cpf, false, 1>(a);
+        case QS_PF8P: return multi ? vl_idx<ModePF, pf, true, 2>(a) : vl_idx<ModePF, pf, false, 2>(a);
+        case QS_CPF8P: return multi ? vl_idx<ModePF, cpf, true, 2>(a) : vl_idx<ModePF, cpf, false, 2>(a);
+        default: return QS_ERR_ARG;
+        }
+    }
+    if (a.btype == QS_C64) {
         if (a.dtype == QS_F32) return multi ? vl_idx<ModeF32, float, true>(a) : vl_idx<ModeF32, float, false>(a);
         if (a.dtype == QS_C64)
             return multi ? vl_idx<ModeF32, cx<float>, true>(a) : vl_idx<ModeF32, cx<float>, false>(a);

@@ -1,0 +1,153 @@
+// Conversions to float pairs without FP64 instructions, and row sums with the
+// vectors across the lanes, for the float-instruction sparse kernels
+// (csrc/spmv_lp.cu, csrc/expm_lp.cu, csrc/expm_vl.cu).
+#pragma once
+#include <type_traits>
+#include "lp_modes.cuh"
+
+namespace {
+
+// The pair of x 2^-k rounded to nearest, bit for bit pf_from_double(x 2^-k):
+// the high part is the top 24 significant bits rounded, the low part the signed
+// rest (at most 2^28 units of x's last place) as an integer conversion and a
+// multiplication by a power of two.  One conversion instruction and no FP64:
+// the FP64 form takes five, at a sixty-fourth of the integer rate.  Zeros are
+// their own pair; values whose low part would leave the normal float range
+// (and infinities and NaN) take the FP64 form.
+__device__ __forceinline__ pf pair_rn_scaled(double x, int k)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    const int E = (int)((hi >> 20) & 0x7ffu), ef = E - 896 - k;
+    if (E == 0 || E == 0x7ff || (unsigned)(ef - 54) >= 200u) {
+        if (((hi << 1) | lo) == 0u) return pf{__uint_as_float(hi), 0.f};
+        return pf_from_double(x * pow2(-k));
+    }
+    const uint32_t rest = lo & 0x1fffffffu;
+    const bool up = rest + ((lo >> 29) & 1u) > 0x10000000u;      // to nearest, ties to even
+    const uint32_t h = ((hi & 0x80000000u) | ((uint32_t)ef << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29)) + (up ? 1u : 0u);
+    int r = (int)rest - (up ? 0x20000000 : 0);
+    if (hi & 0x80000000u) r = -r;
+    return pf{__uint_as_float(h), __fmul_rn(__int2float_rn(r), __uint_as_float((uint32_t)(ef - 52) << 23))};
+}
+
+// x 2^-k in the storage of a mode
+template <class M> __device__ __forceinline__ typename M::S scaled_from_double(double x, int k);
+template <> __device__ __forceinline__ pf scaled_from_double<ModePF>(double x, int k) { return pair_rn_scaled(x, k); }
+template <> __device__ __forceinline__ float scaled_from_double<ModeF32>(double x, int k) { return (float)(x * pow2(-k)); }
+
+__device__ __forceinline__ pf shfl_pair(pf a, int src)
+{
+    return pf{__shfl_sync(0xffffffffu, a.h, src & 31), __shfl_sync(0xffffffffu, a.l, src & 31)};
+}
+
+// real value times real x
+template <class M>
+__device__ __forceinline__ void rmul_acc(typename M::S &ar, typename M::S &, typename M::S d, typename M::S x)
+{
+    M::fma(ar, d, x);
+}
+// complex value times real x
+template <class M>
+__device__ __forceinline__ void rmul_acc(typename M::S &ar, typename M::S &ai, const cx<typename M::S> &d,
+                                         typename M::S x)
+{
+    M::fma(ar, d.re, x);
+    M::fma(ai, d.im, x);
+}
+
+// Lane groups of the many-vector kernels: VL lanes own a row, 32 / VL rows to
+// a warp; lanes left over own none.  The vectors are swept at most eight at a
+// time in sweeps of equal width, so few lanes go without one (13 vectors: two
+// sweeps of 7).
+static inline int vl_lanes(int64_t nvec)
+{
+    const int64_t sweeps = (nvec + 7) / 8;
+    return (int)((nvec + sweeps - 1) / sweeps);
+}
+
+constexpr int VB = 4;      // nonzeros of a row in flight
+
+// One batch of VB nonzeros of a row for one vector, the column words in cur
+// (WPL per lane of the group, whose first lane is lane0), entry k the first.
+// FULL: all of them belong to the row; otherwise only the first `left`.  A
+// word past the row's end is zero and its gather reads column 0: an address
+// without a predicate, its product is skipped.
+template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool FULL>
+__device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, const DV *__restrict__ data,
+                                         const uint8_t *__restrict__ codes, const DV *tab,
+                                         const char *__restrict__ x, uint32_t stride, IT k, int left,
+                                         typename M::S (&ar)[2], typename M::S (&ai)[2])
+{
+    using XE = typename std::conditional<XC, typename M::BE, typename M::S>::type;
+    XE xe[VB];
+    DV d[VB];
+#pragma unroll
+    for (int u = 0; u < VB; u++) {
+        const uint32_t w = __shfl_sync(0xffffffffu, cur[u % WPL], lane0 + u / WPL);
+        if constexpr (VMODE == 2) d[u] = tab[w & 255u];
+        const XE *p = reinterpret_cast<const XE *>(x + (uint64_t)(VMODE == 2 ? w >> 8 : w) * stride);
+        if constexpr (XC) xe[u] = M::ldB(p);
+        else xe[u] = M::ldS(p);
+        if constexpr (VMODE == 0) d[u] = FULL || u < left ? ldv(data + k + u) : vzero<DV>();
+        if constexpr (VMODE == 1) d[u] = tab[FULL || u < left ? (uint32_t)__ldcs(codes + k + u) : 0u];
+    }
+#pragma unroll
+    for (int u = 0; u < VB; u++) {
+        if (FULL || u < left) {
+            if constexpr (XC) vmul_acc<M>(ar[u & 1], ai[u & 1], d[u], xe[u]);
+            else rmul_acc<M>(ar[u & 1], ai[u & 1], d[u], xe[u]);
+        }
+    }
+}
+
+// Sum of one row for one vector, with the vectors across the lanes: a group
+// of VL lanes owns a row and lane v of it vector c, so one warp load gathers
+// the VL vectors' entries of a nonzero as one contiguous piece.  The group's
+// column words are loaded VB at a time, WPL per lane (one, or two where VL is 2
+// or 3), a batch ahead of their use, and handed round by shuffles.  The loop is
+// bound by its instruction count (issue slots 73% busy in the product with 8
+// vectors), nearly all of it float-pair arithmetic: batches that every row of
+// the warp fills run without predicates, addresses are one 32 x 32
+// multiply-add, and lanes past the last vector (c clamped by the caller) load
+// and compute like the rest.  Every lane of the warp calls it with its row's
+// range (empty for none; owns: the lane belongs to a row group).  x: the vectors' base at vector c; stride: bytes per
+// row of vectors.  VMODE: 0 one value per nonzero, 1 coded, 2 codes packed into
+// the column words (tab: the 256 values).
+template <class M, class DV, bool XC, class IT, int VMODE, int WPL>
+__device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, const DV *__restrict__ data,
+                                           const uint8_t *__restrict__ codes, const DV *tab, const void *x,
+                                           uint32_t stride, int v, int lane0, bool owns, IT k0, IT k1,
+                                           typename M::S &sr, typename M::S &si)
+{
+    const int len = (int)(k1 - k0);
+    const int most = __reduce_max_sync(0xffffffffu, len);
+    const int least = __reduce_min_sync(0xffffffffu, owns ? len : most);     // of the lanes that own a row
+    const char *xb = reinterpret_cast<const char *>(x);
+    const bool loads = v * WPL < VB;           // the lanes that fetch the words
+    uint32_t word[WPL];
+    auto fetch = [&](int b) {
+#pragma unroll
+        for (int i = 0; i < WPL; i++) {
+            const int at = b + v * WPL + i;
+            word[i] = loads && at < len ? (uint32_t)__ldcs(indices + k0 + at) : 0u;
+        }
+    };
+    // even and odd places apart, as two lanes of a row hand-out: half the
+    // roundings that one chain collects
+    typename M::S ar[2] = {M::zero(), M::zero()}, ai[2] = {M::zero(), M::zero()};
+    fetch(0);
+    for (int b = 0; b < most; b += VB) {
+        uint32_t cur[WPL];
+#pragma unroll
+        for (int i = 0; i < WPL; i++) cur[i] = word[i];
+        fetch(b + VB);
+        if (b + VB <= least)
+            vl_batch<M, DV, XC, IT, VMODE, WPL, true>(cur, lane0, data, codes, tab, xb, stride, k0 + b, VB, ar, ai);
+        else
+            vl_batch<M, DV, XC, IT, VMODE, WPL, false>(cur, lane0, data, codes, tab, xb, stride, k0 + b, len - b, ar, ai);
+    }
+    sr = M::merge(ar[0], ar[1]);
+    si = M::merge(ai[0], ai[1]);
+}
+
+}  // namespace

@@ -13,32 +13,18 @@
 //   * single precision (qs_csr_matvec with float32 / complex64 x and values):
 //     FP32 products and row sums, float32 / complex64 y.
 //
-// Row hand-out, lanes per row and entries in flight follow csrc/sparse.cu;
-// after the butterfly reduction lanes 0 and 1 of a row group write the real
-// and imaginary part of y.
+// One vector: row hand-out, lanes per row and entries in flight follow
+// csrc/sparse.cu; after the butterfly reduction lanes 0 and 1 of a row group
+// write the real and imaginary part of y.  Several vectors: the vectors
+// across the lanes.
 #include "qs_common.cuh"
 #include "pairf.cuh"
-#include "lp_modes.cuh"
+#include "lp_lanes.cuh"
 
 namespace {
 
 template <class T> struct is_cx { static constexpr bool value = false; };
 template <class S> struct is_cx<cx<S>> { static constexpr bool value = true; };
-
-// real value times real x
-template <class M>
-__device__ __forceinline__ void rmul_acc(typename M::S &ar, typename M::S &, typename M::S d, typename M::S x)
-{
-    M::fma(ar, d, x);
-}
-// complex value times real x
-template <class M>
-__device__ __forceinline__ void rmul_acc(typename M::S &ar, typename M::S &ai, const cx<typename M::S> &d,
-                                         typename M::S x)
-{
-    M::fma(ar, d.re, x);
-    M::fma(ai, d.im, x);
-}
 
 // output stores: YT double / float (real) or cdbl / cflt (complex)
 template <class M> __device__ __forceinline__ void st_out(double *y, int64_t e, int, typename M::S v, int k, int ow)
@@ -74,11 +60,11 @@ template <class M> __device__ __forceinline__ void st_out(cflt *y, int64_t e, in
 // QS_CPF8P); 3 packed, one complex vector, the column words read four per
 // 16-byte load (indices readable up to the next multiple of four words).
 // The table is staged in shared memory.
-template <class M, class DV, bool XC, class YT, class IT, int NB, int U, int VM>
+template <class M, class DV, bool XC, class YT, class IT, int U, int VM>
 __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const IT *__restrict__ indptr,
                                                       const int32_t *__restrict__ indices,
                                                       const DV *__restrict__ data, const void *__restrict__ xv,
-                                                      YT *__restrict__ y, int64_t nvec, cdbl a, int overwrite,
+                                                      YT *__restrict__ y, cdbl a, int overwrite,
                                                       const unsigned long long *__restrict__ xnorm)
 {
     using S = typename M::S;
@@ -115,29 +101,26 @@ __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const 
         const bool valid = r < n;
         const bool writer = valid && (COUT ? lane < 2 : lane == 0);
         const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
-        for (int64_t c0 = 0; c0 < nvec; c0 += NB) {
-            S ar[NB], ai[NB];
+        S ar = M::zero(), ai = M::zero();
+        if constexpr (VM == 3) {
+            // the row's packed column words in 16-byte aligned groups of four,
+            // group g of the row to lane g mod G
+            for (IT c = (k0 & ~(IT)3) + 4 * lane; c < k1; c += (IT)(4 * G)) {
+                const uint4 w4 = __ldcs(reinterpret_cast<const uint4 *>(indices + c));
+                const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-            for (int b = 0; b < NB; b++) ar[b] = ai[b] = M::zero();
-            if constexpr (VM == 3) {
-                // one vector: the row's packed column words in 16-byte aligned
-                // groups of four, group g of the row to lane g mod G
-                for (IT c = (k0 & ~(IT)3) + 4 * lane; c < k1; c += (IT)(4 * G)) {
-                    const uint4 w4 = __ldcs(reinterpret_cast<const uint4 *>(indices + c));
-                    const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+                for (int h = 0; h < 4; h += 2) {
+                    BE bv[2];
 #pragma unroll
-                    for (int h = 0; h < 4; h += 2) {
-                        BE bv[2];
+                    for (int i = 0; i < 2; i++)
+                        bv[i] = (c + h + i >= k0 && c + h + i < k1) ? M::ldB(xc + (int32_t)(w[h + i] >> 8), keep)
+                                                                    : BE{M::zero(), M::zero()};
 #pragma unroll
-                        for (int i = 0; i < 2; i++)
-                            bv[i] = (c + h + i >= k0 && c + h + i < k1) ? M::ldB(xc + (int32_t)(w[h + i] >> 8), keep)
-                                                                        : BE{M::zero(), M::zero()};
-#pragma unroll
-                        for (int i = 0; i < 2; i++)
-                            if (c + h + i >= k0 && c + h + i < k1) vmul_acc<M>(ar[0], ai[0], s_tab[w[h + i] & 255u], bv[i]);
-                    }
+                    for (int i = 0; i < 2; i++)
+                        if (c + h + i >= k0 && c + h + i < k1) vmul_acc<M>(ar, ai, s_tab[w[h + i] & 255u], bv[i]);
                 }
-            } else {
+            }
+        } else {
             for (IT k = k0 + lane; k < k1; k += (IT)(G * U)) {
                 int32_t col[U];
                 DV d[U];
@@ -158,63 +141,127 @@ __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const 
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     if (k + (IT)(u * G) < k1) {
-#pragma unroll
-                        for (int b = 0; b < NB; b++) {
-                            if (NB == 1 || c0 + b < nvec) {
-                                const int64_t xi = (int64_t)col[u] * nvec + c0 + b;
-                                if constexpr (XC)
-                                    vmul_acc<M>(ar[b], ai[b], d[u], NB == 1 ? M::ldB(xc + xi, keep) : M::ldB(xc + xi));
-                                else rmul_acc<M>(ar[b], ai[b], d[u], M::ldS(xr + xi));
-                            }
-                        }
+                        if constexpr (XC) vmul_acc<M>(ar, ai, d[u], M::ldB(xc + col[u], keep));
+                        else rmul_acc<M>(ar, ai, d[u], M::ldS(xr + col[u]));
                     }
                 }
             }
+        }
+        for (int o = G >> 1; o > 0; o >>= 1) {
+            ar = M::merge(ar, M::shfl_xor(ar, o));
+            if constexpr (COUT) ai = M::merge(ai, M::shfl_xor(ai, o));
+        }
+        if (writer) {
+            const S accr = M::fin(ar);
+            if constexpr (COUT) {
+                const S acci = M::fin(ai);
+                const S v = comp ? M::add(M::mul(av.re, acci), M::mul(av.im, accr))
+                                 : M::sub(M::mul(av.re, accr), M::mul(av.im, acci));
+                st_out<M>(y, r, comp, v, k2, overwrite);
+            } else {
+                st_out<M>(y, r, 0, M::mul(av.re, accr), k2, overwrite);
             }
-#pragma unroll
-            for (int b = 0; b < NB; b++) {
-                for (int o = G >> 1; o > 0; o >>= 1) {
-                    ar[b] = M::merge(ar[b], M::shfl_xor(ar[b], o));
-                    if constexpr (COUT) ai[b] = M::merge(ai[b], M::shfl_xor(ai[b], o));
-                }
-            }
-            if (writer) {
-#pragma unroll
-                for (int b = 0; b < NB; b++) {
-                    if (c0 + b >= nvec) break;
-                    const int64_t e = r * nvec + c0 + b;
-                    const S accr = M::fin(ar[b]);
-                    if constexpr (COUT) {
-                        const S acci = M::fin(ai[b]);
-                        const S v = comp ? M::add(M::mul(av.re, acci), M::mul(av.im, accr))
-                                         : M::sub(M::mul(av.re, accr), M::mul(av.im, acci));
-                        st_out<M>(y, e, comp, v, k2, overwrite);
-                    } else {
-                        st_out<M>(y, e, 0, M::mul(av.re, accr), k2, overwrite);
-                    }
+        }
+    }
+}
+
+// Several vectors: the vectors across the lanes (vl_row_sum), VL lanes to a
+// row, sweeps of VL vectors.  With the vectors on the accumulators of one lane
+// instead, a warp's load of one vector touches 32 lines for 32 nonzeros and is
+// bound by the L1 tag rate.  Measured (whole product, x split included), the
+// Ising chain L = 22 at k != 0 (191 k rows, 4.4 M complex nonzeros): 8 vectors
+// 194 us then, 120 us now; 5 vectors 112 / 87 us; J1-J2 L = 28 (361 k rows,
+// 10.7 M real nonzeros): 8 vectors 401 / 191 us, 2 vectors 98 / 69 us.  Complex
+// pairs run at three blocks per SM (four spill: 129 us), the rest at four.
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL>
+__global__ void __launch_bounds__(256, std::is_same<DV, cpf>::value ? 3 : 4)
+spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices,
+               const DV *__restrict__ data, const void *__restrict__ xv, YT *__restrict__ y, int64_t nvec, int VL,
+               cdbl a, int overwrite, const unsigned long long *__restrict__ xnorm)
+{
+    using S = typename M::S;
+    using XE = typename std::conditional<XC, typename M::BE, S>::type;
+    constexpr bool COUT = XC || is_cx<DV>::value;
+    __shared__ S s_a[2];
+    __shared__ int s_k;
+    if (threadIdx.x == 0) s_a[0] = M::from_d(a.x);
+    if (threadIdx.x == 1) s_a[1] = M::from_d(a.y);
+    if (threadIdx.x == 2) s_k = xnorm ? scale_exp(__longlong_as_double((long long)*xnorm)) : 0;
+    constexpr bool CODED = VM != 0;
+    __shared__ DV s_tab[CODED ? QS_CODE_TABLE : 1];
+    const uint8_t *codes = nullptr;
+    if constexpr (CODED) {
+        for (int i = threadIdx.x; i < QS_CODE_TABLE; i += blockDim.x) s_tab[i] = ldv(data + i);
+        codes = reinterpret_cast<const uint8_t *>(data + QS_CODE_TABLE);
+    }
+    __syncthreads();
+    const cx<S> av{s_a[0], s_a[1]};
+    const int k2 = s_k;
+    const int RPW = 32 / VL, grp = (threadIdx.x & 31) / VL, lane0 = grp * VL, v = (threadIdx.x & 31) - lane0;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t rb = warp * RPW; rb < n; rb += nwarps * RPW) {
+        const int64_t r = rb + grp;
+        const bool valid = r < n && grp < RPW;
+        const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
+        for (int64_t c0 = 0; c0 < nvec; c0 += VL) {
+            const int64_t c = c0 + v < nvec ? c0 + v : nvec - 1;
+            const bool act = valid && c0 + v < nvec;
+            S ar = M::zero(), ai = M::zero();
+            vl_row_sum<M, DV, XC, IT, VM, WPL>(indices, data, codes, s_tab, reinterpret_cast<const XE *>(xv) + c,
+                                               (uint32_t)(nvec * sizeof(XE)), v, lane0, grp < RPW, k0, k1, ar, ai);
+            if (act) {
+                const int64_t e = r * nvec + c;
+                const S accr = M::fin(ar);
+                if constexpr (COUT) {
+                    const S acci = M::fin(ai);
+                    st_out<M>(y, e, 0, M::sub(M::mul(av.re, accr), M::mul(av.im, acci)), k2, overwrite);
+                    st_out<M>(y, e, 1, M::add(M::mul(av.re, acci), M::mul(av.im, accr)), k2, overwrite);
+                } else {
+                    st_out<M>(y, e, 0, M::mul(av.re, accr), k2, overwrite);
                 }
             }
         }
     }
 }
 
-// largest |component| of a double array into *norm (bits of a double >= 0)
-__global__ void xnorm_kernel(int64_t count, const double *__restrict__ x, unsigned long long *norm)
+// The power of two at the largest |component| of a double array, as the high
+// word of a double in *norm (scale_exp reads its exponent only).  Integer
+// compares of the high words: an FP64 maximum is two FP64-pipe instructions.
+// NaN counts as nothing, as in an FP64 maximum.
+__global__ void __launch_bounds__(256) xnorm_kernel(int64_t count, const double *__restrict__ x,
+                                                    unsigned long long *norm)
 {
-    double m = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
-        m = fmax(m, fabs(__ldcs(x + i)));
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(norm, (unsigned long long)__double_as_longlong(m));
+    uint32_t m = 0;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) {
+        const double v = __ldg(x + i);
+        uint32_t h = (uint32_t)__double2hiint(v) & 0x7fffffffu;
+        if (h >= 0x7ff00000u && (h > 0x7ff00000u || __double2loint(v) != 0)) h = 0u;
+        m = h > m ? h : m;
+    }
+    // one atomic per block: all of them meet at one address
+    __shared__ uint32_t s_m[8];
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        m = __reduce_max_sync(0xffu, s_m[threadIdx.x]);
+        if (threadIdx.x == 0 && m) atomicMax(norm, (unsigned long long)m << 32);
+    }
 }
 
 // xs[i] = pair(x[i] 2^-k), k from *norm
-__global__ void xsplit_kernel(int64_t count, const double *__restrict__ x, float2 *__restrict__ xs,
-                              const unsigned long long *__restrict__ norm)
+__global__ void __launch_bounds__(256) xsplit_kernel(int64_t count, const double *__restrict__ x,
+                                                     float2 *__restrict__ xs,
+                                                     const unsigned long long *__restrict__ norm)
 {
-    const double sc = pow2(-scale_exp(__longlong_as_double((long long)*norm)));
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        const pf v = pf_from_double(__ldcs(x + i) * sc);
+    const int k = scale_exp(__longlong_as_double((long long)*norm));
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) {
+        const pf v = pair_rn_scaled(__ldcs(x + i), k);
         xs[i] = make_float2(v.h, v.l);
     }
 }
@@ -243,17 +290,31 @@ static int grid_rows(int64_t n, int G)
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-template <class M, class DV, bool XC, class YT, class IT, int NB, int U, int VM>
+template <class M, class DV, bool XC, class YT, class IT, int U, int VM>
 int spmv_go(const SpmvArgs &a)
 {
     int lg = 0;
     while ((1 << lg) < a.G) lg++;
     // persistent grid (grid-stride kernel): one wave of resident blocks
     static int resident = 0;
-    auto k = spmv_lp_kernel<M, DV, XC, YT, IT, NB, U, VM>;
+    auto k = spmv_lp_kernel<M, DV, XC, YT, IT, U, VM>;
     const int blocks = qs_persistent_grid(k, 256, grid_rows(a.n, a.G), resident);
-    k<<<blocks, 256, 0, a.st>>>(a.n, lg, (const IT *)a.indptr, a.indices, (const DV *)a.data, a.x, (YT *)a.y,
-                                a.nvec, a.a, a.overwrite, a.xnorm);
+    k<<<blocks, 256, 0, a.st>>>(a.n, lg, (const IT *)a.indptr, a.indices, (const DV *)a.data, a.x, (YT *)a.y, a.a,
+                                a.overwrite, a.xnorm);
+    QS_CHECK(cudaGetLastError());
+    return QS_OK;
+}
+
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL>
+int spmm_go(const SpmvArgs &a)
+{
+    static int resident = 0;
+    auto k = spmm_vl_kernel<M, DV, XC, YT, IT, VM, WPL>;
+    const int VL = vl_lanes(a.nvec);
+    const int64_t rows = 8 * (32 / VL);       // per block and sweep
+    const int blocks = qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident);
+    k<<<blocks, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, a.x, (YT *)a.y, a.nvec, VL,
+                                a.a, a.overwrite, a.xnorm);
     QS_CHECK(cudaGetLastError());
     return QS_OK;
 }
@@ -263,18 +324,17 @@ int spmv_nb(const SpmvArgs &a)
 {
     if constexpr (VM == 3) {
         if (a.nvec != 1 || !XC) return QS_ERR_ARG;
-        return spmv_go<M, DV, XC, YT, IT, 1, 1, 3>(a);
+        return spmv_go<M, DV, XC, YT, IT, 1, 3>(a);
     } else {
-    if (a.nvec == 1) {
-        if constexpr (sizeof(IT) == 4) {
-            if (a.U >= 4) return spmv_go<M, DV, XC, YT, IT, 1, 4, VM>(a);
-            if (a.U >= 2) return spmv_go<M, DV, XC, YT, IT, 1, 2, VM>(a);
+        if (a.nvec == 1) {
+            if constexpr (sizeof(IT) == 4) {
+                if (a.U >= 4) return spmv_go<M, DV, XC, YT, IT, 4, VM>(a);
+                if (a.U >= 2) return spmv_go<M, DV, XC, YT, IT, 2, VM>(a);
+            }
+            return spmv_go<M, DV, XC, YT, IT, 1, VM>(a);
         }
-        return spmv_go<M, DV, XC, YT, IT, 1, 1, VM>(a);
-    }
-    if (a.nvec == 2) return spmv_go<M, DV, XC, YT, IT, 2, 1, VM>(a);
-    if (a.nvec <= 4) return spmv_go<M, DV, XC, YT, IT, 4, 1, VM>(a);
-    return spmv_go<M, DV, XC, YT, IT, 8, 1, VM>(a);
+        if (a.nvec <= 3) return spmm_go<M, DV, XC, YT, IT, VM, 2>(a);
+        return spmm_go<M, DV, XC, YT, IT, VM, 1>(a);
     }
 }
 
@@ -320,7 +380,7 @@ extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, i
                                    double a_re, double a_im, int overwrite, int group, void *xs, void *norm,
                                    void *stream)
 {
-    if (n < 0 || nvec < 1 || (n > 0 && (!indptr || !x || !y || !xs || !norm))) return QS_ERR_ARG;
+    if (n < 0 || nvec < 1 || nvec >= (1 << 27) || (n > 0 && (!indptr || !x || !y || !xs || !norm))) return QS_ERR_ARG;
     if (n == 0) return QS_OK;
     const bool xc = xtype == QS_C128;
     if (!xc && xtype != QS_F64) return QS_ERR_ARG;
@@ -341,8 +401,8 @@ extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, i
     const int64_t count = n * nvec * (xc ? 2 : 1);
     QS_CHECK(cudaMemsetAsync(nrm, 0, sizeof(unsigned long long), st));
     int64_t b = (count + 255) / 256, cap = (int64_t)qs_num_sms() * 8;
-    const int blocks = (int)(b > cap ? cap : b);
-    xnorm_kernel<<<blocks, 256, 0, st>>>(count, (const double *)x, nrm);
+    const int blocks = (int)(b > cap ? cap : b), nblk = (int)(b > cap / 2 ? cap / 2 : b);
+    xnorm_kernel<<<nblk, 256, 0, st>>>(count, (const double *)x, nrm);
     xsplit_kernel<<<blocks, 256, 0, st>>>(count, (const double *)x, (float2 *)xs, nrm);
     QS_CHECK(cudaGetLastError());
     SpmvArgs s{n, indptr, idx64, indices, pdata, xs, y, nvec, cdbl{a_re, a_im}, overwrite, nrm, G, U, st};

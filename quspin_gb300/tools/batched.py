@@ -112,7 +112,8 @@ class MultiSectorExpm:
         return list(self._offs)
 
     def _term(self, j, bin_, bout, tol, group):
-        A = self._A
+        from ..tune import lanes_operand
+        A = lanes_operand(self._A, self.nvec, group)
         _lib.call("qs_taylor_multi_term", self.n, D.ptr(A.indptr), D.ptr(A.indices), D.ptr(A.data), A.vcode,
                   D.ptr(bin_), D.ptr(bout), self._btype, D.ptr(self.F), self.nvec, D.ptr(self._soff),
                   D.ptr(self._mu), D.ptr(self._coeff), j, tol, D.ptr(self._ctl), group, D.stream())
@@ -133,8 +134,8 @@ class MultiSectorExpm:
                  if not (self.nvec == 1 and U > 2)]
         codes += [encode(G, U) | (occ << 18) for G, U in occ_candidates(self._A, self.nvec, self._btype)
                   for occ in (1, 2)]
-        if self.nvec > 1:      # the vectors-across-lanes kernel (csrc/expm_vl.cu), three shapes
-            codes += [encode(2, 2) | (shape << 20) for shape in (1, 2, 3)]
+        if self.nvec > 1:      # the vectors-across-lanes kernel (csrc/expm_vl.cu)
+            codes += [encode(2, 2) | (1 << 20)]
         for code in codes:
             self._ctl.copy_(self._ctl_tmpl)
             t = _time(lambda: self._term(0, b0, b1, 0.0, code))

@@ -319,8 +319,9 @@ class ExpmMultiplyParallel:
         cf = consts[:max(m, 1)]
         etap = consts[max(m, 1):max(m, 1) + 1]
         onep = consts[max(m, 1) + 1:]
-        from ..tune import tune_taylor
+        from ..tune import lanes_operand, tune_taylor
         group = tune_taylor(M, nvec, btype)
+        M = lanes_operand(M, nvec, group)
         rown = self._rownorm(n) if (btype != _lib.C128 and nvec > 8) else None
         _lib.call("qs_expm_multiply_rows", n, M.nnz, D.ptr(M.indptr), M.idx64, D.ptr(M.indices), D.ptr(M.data),
                   M.vcode, D.ptr(F), nvec, s, m, tol, mu.real, mu.imag, D.ptr(cf), D.ptr(etap),

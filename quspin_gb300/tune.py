@@ -58,6 +58,18 @@ def r32_candidates(M, nvec, btype):
     return cands
 
 
+def lanes_operand(M, nvec, code):
+    """The operand a launch code reads: with the vectors across the lanes
+    (several vectors, shape bits set or code 0) a coded operand's packed form
+    where it has one -- a word per nonzero instead of an index and a code
+    byte; otherwise M itself."""
+    if nvec == 1 or not getattr(M, "coded", False) or (code and not (code >> 20) & 7):
+        return M
+    pack = getattr(M, "packed", None)
+    P = pack() if pack is not None else None
+    return M if P is None else P
+
+
 def _time(fn, reps=5):
     st = torch.cuda.current_stream()
     for _ in range(2):
@@ -80,7 +92,9 @@ def tune_spmv(M, nvec=1, xdtype=np.complex128, precision="double", operand=None)
     if key in cache:
         return cache[key]
     n = M.shape[0]
-    if n < MIN_ROWS or getattr(M, "idx64", 0):
+    if n < MIN_ROWS or getattr(M, "idx64", 0) or (nvec > 1 and precision == "double"):
+        # several vectors in the float forms have one shape, the vectors
+        # across the lanes (csrc/spmv_lp.cu)
         cache[key] = 0
         return 0
     shape = (n,) if nvec == 1 else (n, nvec)
@@ -125,18 +139,18 @@ def tune_taylor(M, nvec, btype):
         rown = torch.empty(2 * n, dtype=torch.float64, device=D.device())
     cands += [(G, U, occ << 2) for G, U in occ_candidates(M, nvec, btype) for occ in (1, 2)]
     if nvec > 1 and btype != _lib.C128:
-        # the vectors-across-lanes kernel (csrc/expm_vl.cu), three shapes
-        cands += [(2, 2, shape << 4) for shape in (1, 2, 3)]
+        cands += [(2, 2, 1 << 4)]     # the vectors-across-lanes kernel (csrc/expm_vl.cu)
     if getattr(M, "vcode", None) in (_lib.PF8P, _lib.CPF8P):
         cands = []                 # the packed form runs only in the single-vector kernels
     cands += [({1: 4, 2: 2, 3: 8, 4: 2, 5: 4, 6: 2, 7: 4}[shape], 2, (shape << 4) | (occ << 2))
               for shape, occ in r32_candidates(M, nvec, btype)]
     for G, U, ch in cands:
         code = encode(G, U) | (ch << 16)
+        A = lanes_operand(M, nvec, code)
 
         def run():
-            _lib.call("qs_taylor_term_rows", n, M.nnz, D.ptr(M.indptr), M.idx64, D.ptr(M.indices), D.ptr(M.data),
-                      M.vcode, D.ptr(b0), D.ptr(b1), btype, D.ptr(F), nvec, 0.0, 0.0, D.ptr(coeff), 0, 0.0,
+            _lib.call("qs_taylor_term_rows", n, A.nnz, D.ptr(A.indptr), A.idx64, D.ptr(A.indices), D.ptr(A.data),
+                      A.vcode, D.ptr(b0), D.ptr(b1), btype, D.ptr(F), nvec, 0.0, 0.0, D.ptr(coeff), 0, 0.0,
                       D.ptr(ctl), code, D.ptr(rown), D.stream())
         t = _time(run)
         if best_t is None or t < best_t:
