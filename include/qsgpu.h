@@ -282,6 +282,17 @@ int qs_lanczos_reorth(int64_t n, int cplx, int nk, const double *d_Q, int64_t ld
                       double *d_scratch, void *d_ctl, void *stream);
 int qs_lanczos_reorth_adaptive(int64_t n, int cplx, int nk, const double *d_Q, int64_t ldq, double *d_r,
                                int max_passes, double *d_scratch, void *d_ctl, void *stream);
+/* A whole m-step run on a float-pair CSR (pdtype 4 / 5, or packed 8 / 9; int32
+ * d_indptr) with the vectors kept in d_Q [m, n] (row 0 the normalised start
+ * vector): three launches per step, or six to nine with reorth.  d_r: n
+ * elements; d_xs: n split elements; d_ab: a[m], b[m]; d_ctl:
+ * qs_lanczos_run_ctl_bytes() of zeros, its second int32 set to m (on return:
+ * the number of valid vectors). */
+int qs_lanczos_run_ctl_bytes(void);
+int64_t qs_lanczos_run_scratch_doubles(int m, int reorth);
+int qs_lanczos_run(int64_t n, int m, int cplx, double eps, int reorth, const int32_t *d_indptr,
+                   const int32_t *d_indices, const void *d_pdata, int pdtype, int group, double *d_Q, double *d_r,
+                   void *d_xs, double *d_ab, double *d_scratch, void *d_ctl, void *stream);
 int qs_lanczos_lincomb(int64_t n_el, int nk, const double *d_c, int cplx_c, const double *d_Q, int64_t ldq,
                        int cplx_q, double *d_out, void *stream);
 

@@ -12,14 +12,11 @@
 // against all previous Lanczos vectors, stored row-major in Q[m, n]) runs
 // between the a[i] and b[i] steps.
 #include "qs_common.cuh"
+#include "lp_lanes.cuh"
+#include "lanczos.cuh"
 
 #define LZ_THREADS 256
 #define LZ_BLOCKS_MAX 1024
-
-struct LzCtl {
-    int done;      // b[i] < eps was seen
-    int m_eff;     // number of valid Lanczos vectors
-};
 
 extern "C" int qs_lanczos_ctl_bytes() { return (int)sizeof(LzCtl); }
 extern "C" int qs_lanczos_scratch_doubles() { return 2 * LZ_BLOCKS_MAX; }
@@ -32,26 +29,19 @@ static int lz_blocks(int64_t n)
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-__device__ __forceinline__ double wsum(double v)
+// x / b with b's reciprocal at hand: one correction step on the exact
+// remainder, three FP64 instructions where a division takes about ten.  `fast`
+// says that b and its reciprocal are well inside the normal range.
+__device__ __forceinline__ double div_by(double x, double b, double inv, bool fast)
 {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
+    if (!fast) return x / b;
+    const double q = x * inv;
+    return fma(fma(-q, b, x), inv, q);
 }
-
-__device__ __forceinline__ double block_sum(double v)
+__device__ __forceinline__ bool div_fast(double b)
 {
-    __shared__ double sh[32];
-    v = wsum(v);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (w == 0) {
-        t = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-        t = wsum(t);
-    }
-    return t;   // valid in thread 0
+    const int e = (__double2hiint(b) >> 20) & 0x7ff;
+    return e > 123 && e < 1923;
 }
 
 // q = r / b[i-1] (also the first step with b = norm of v0 when i == 0)
@@ -59,9 +49,57 @@ __global__ void lz_scale_kernel(int64_t n2, const double *__restrict__ r, const 
                                 double *__restrict__ q, const LzCtl *ctl)
 {
     if (ctl && ctl->done) return;
-    const double b = *bptr;
+    const double b = *bptr, inv = 1.0 / b;
+    const bool fast = div_fast(b);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += (int64_t)gridDim.x * blockDim.x)
-        q[i] = r[i] / b;
+        q[i] = div_by(r[i], b, inv, fast);
+}
+
+// The same (b null: q stays as it is), and q as float pairs in xs for the
+// product of a whole run (csrc/spmv_lp.cu).  A normalised vector's largest
+// component lies between 1 / sqrt(n) and 1, so the pairs take a fixed scale
+// 2^xexp and no pass over q for its norm.
+__global__ void __launch_bounds__(LZ_THREADS) lz_scale_split_kernel(int64_t n2, const double *__restrict__ r,
+                                                                    const double *__restrict__ bptr,
+                                                                    double *__restrict__ q, float2 *__restrict__ xs,
+                                                                    int xexp, const LzRunCtl *ctl)
+{
+    if (ctl->done) return;
+    const double b = bptr ? *bptr : 1.0, inv = 1.0 / b;
+    const bool fast = div_fast(b);
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += step) {
+        double x;
+        if (bptr) {
+            x = div_by(r[i], b, inv, fast);
+            q[i] = x;
+        } else {
+            x = q[i];
+        }
+        const pf p = pair_rn_scaled(x, -xexp);
+        xs[i] = make_float2(p.h, p.l);
+    }
+}
+
+// r -= a q, and the sum of |r|^2 finished as `what` says
+__global__ void __launch_bounds__(LZ_THREADS) lz_axpy_run_kernel(int64_t n2, double *__restrict__ r,
+                                                                 const double *__restrict__ aptr,
+                                                                 const double *__restrict__ q, double *partial,
+                                                                 double *out, int what, double eps, int i,
+                                                                 double *state, LzRunCtl *ctl)
+{
+    if (ctl->done) return;
+    const double a = *aptr;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    double s = 0.0;
+#pragma unroll 4
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n2; k += step) {
+        const double x = fma(-a, q[k], r[k]);
+        r[k] = x;
+        s = fma(x, x, s);
+    }
+    lz_block_finish(s, partial, out, what, eps, i, state, ctl);
 }
 
 // r -= b * v (if v) ; partial[blk] = sum Re(conj(q) r)
@@ -180,8 +218,9 @@ lz_gemv_t_kernel(int64_t n, int nk, const double *__restrict__ Q, int64_t ldq, c
                 for (int t = 0; t < R; t++) {
                     if (t < rows) {
                         const double qr = q0[t * ldq + 2 * i], qi = q0[t * ldq + 2 * i + 1];
-                        acc[2 * t] += qr * rr + qi * ri;
-                        acc[2 * t + 1] += qr * ri - qi * rr;
+                        // two chained FMAs each: the FP64 pipe bounds this kernel
+                        acc[2 * t] = fma(qi, ri, fma(qr, rr, acc[2 * t]));
+                        acc[2 * t + 1] = fma(-qi, rr, fma(qr, ri, acc[2 * t + 1]));
                     }
                 }
             } else {
@@ -224,29 +263,69 @@ __global__ void lz_gemv_t_finish(int nb, int nk, int cplx, const double *__restr
     }
 }
 
+// element i of sum_k h[k] Q[k] (two chained FMAs per real part and row)
+template <bool CPLX>
+__device__ __forceinline__ void lz_row_comb(int64_t i, int nk, const double *__restrict__ Q, int64_t ldq,
+                                            const double *__restrict__ h, double &ar, double &ai)
+{
+    ar = ai = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < nk; k++) {
+        const double *qk = Q + (int64_t)k * ldq;
+        if constexpr (CPLX) {
+            const double qr = qk[2 * i], qi = qk[2 * i + 1], hr = __ldg(h + 2 * k), hi = __ldg(h + 2 * k + 1);
+            ar = fma(-qi, hi, fma(qr, hr, ar));
+            ai = fma(qi, hr, fma(qr, hi, ai));
+        } else {
+            ar = fma(qk[i], __ldg(h + 2 * k), ar);
+        }
+    }
+}
+
 // r -= sum_k h[k] Q[k]
-__global__ void lz_gemv_n_kernel(int64_t n, int cplx, int nk, const double *__restrict__ Q, int64_t ldq,
-                                 const double *__restrict__ h, double *__restrict__ r, const LzCtl *ctl,
-                                 const double *skip)
+template <bool CPLX>
+__global__ void __launch_bounds__(LZ_THREADS)
+lz_gemv_n_kernel(int64_t n, int nk, const double *__restrict__ Q, int64_t ldq, const double *__restrict__ h,
+                 double *__restrict__ r, const LzCtl *ctl, const double *skip)
 {
     if (ctl->done || (skip && *skip != 0.0)) return;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (cplx) {
-            double ar = 0.0, ai = 0.0;
-            for (int k = 0; k < nk; k++) {
-                const double *qk = Q + (int64_t)k * ldq;
-                double qr = qk[2 * i], qi = qk[2 * i + 1], hr = h[2 * k], hi = h[2 * k + 1];
-                ar += qr * hr - qi * hi;
-                ai += qr * hi + qi * hr;
-            }
+        double ar, ai;
+        lz_row_comb<CPLX>(i, nk, Q, ldq, h, ar, ai);
+        if constexpr (CPLX) {
             r[2 * i] -= ar;
             r[2 * i + 1] -= ai;
         } else {
-            double a = 0.0;
-            for (int k = 0; k < nk; k++) a += Q[(int64_t)k * ldq + i] * h[2 * k];
-            r[i] -= a;
+            r[i] -= ar;
         }
     }
+}
+
+// The same in a whole run, with the norm that decides on another pass and is
+// the step's b (LZ_PASS): a pass over r less than a norm kernel of its own.
+template <bool CPLX>
+__global__ void __launch_bounds__(LZ_THREADS)
+lz_gemv_n_run_kernel(int64_t n, int nk, const double *__restrict__ Q, int64_t ldq, const double *__restrict__ h,
+                     double *__restrict__ r, double *partial, double *out, double eps, int step, double *state,
+                     int again, LzRunCtl *ctl)
+{
+    if (ctl->done || (again && state[1] != 0.0)) return;
+    double s = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double ar, ai;
+        lz_row_comb<CPLX>(i, nk, Q, ldq, h, ar, ai);
+        if constexpr (CPLX) {
+            const double x = r[2 * i] - ar, y = r[2 * i + 1] - ai;
+            r[2 * i] = x;
+            r[2 * i + 1] = y;
+            s = fma(y, y, fma(x, x, s));
+        } else {
+            const double x = r[i] - ar;
+            r[i] = x;
+            s = fma(x, x, s);
+        }
+    }
+    lz_block_finish(s, partial, out, LZ_PASS, eps, step, state, ctl);
 }
 
 // q = r / b (b device scalar); skipped once the stopping test fired
@@ -294,11 +373,8 @@ extern "C" int64_t qs_lanczos_reorth_scratch_doubles(int nk)
     return (int64_t)2 * LZ_BLOCKS_MAX * k + 2 * k + 2 + LZ_BLOCKS_MAX;
 }
 
-// Pass control of the adaptive reorthogonalisation.  state[0]: squared norm
-// of r before the last pass; state[1]: 1 once a pass kept at least 1/sqrt(2)
-// of the norm (then r is orthogonal to the rows to working precision and
-// the remaining passes return at once).  first: record the norm of the
-// incoming r and clear the flag.
+// Pass control of the adaptive reorthogonalisation (lz_verdict).  first:
+// record the norm of the incoming r and clear the flag.
 __global__ void lz_dgks_kernel(int nb, const double *__restrict__ partial, double *state, int first, const LzCtl *ctl)
 {
     if (ctl->done) return;
@@ -310,10 +386,8 @@ __global__ void lz_dgks_kernel(int nb, const double *__restrict__ partial, doubl
         if (first) {
             state[0] = s;
             state[1] = 0.0;
-        } else if (s >= 0.5 * state[0]) {
-            state[1] = 1.0;
         } else {
-            state[0] = s;
+            lz_verdict(s, state);
         }
     }
 }
@@ -325,7 +399,8 @@ static void reorth_pass(cudaStream_t st, int nb, int64_t n, int cplx, int nk, co
     else lz_gemv_t_kernel<false><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, ldq, r, part, ctl, skip);
     const int nacc = cplx ? 2 * nk : nk;
     lz_gemv_t_finish<<<(nacc + 7) / 8, 256, 0, st>>>(nb, nk, cplx, part, h, ctl, skip);
-    lz_gemv_n_kernel<<<nb, LZ_THREADS, 0, st>>>(n, cplx, nk, Q, cplx ? 2 * ldq : ldq, h, r, ctl, skip);
+    if (cplx) lz_gemv_n_kernel<true><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, 2 * ldq, h, r, ctl, skip);
+    else lz_gemv_n_kernel<false><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, ldq, h, r, ctl, skip);
 }
 
 // Classical Gram-Schmidt, applied `passes` times: r -= Q[:nk]^T (conj(Q[:nk]) r).
@@ -375,6 +450,72 @@ extern "C" int qs_lanczos_reorth_adaptive(int64_t n, int cplx, int nk, const dou
         }
     }
     QS_CHECK(cudaGetLastError());
+    return QS_OK;
+}
+
+// Scratch of qs_lanczos_run: block partials, pass state, and with reorth the
+// partials and values of the projections on up to m rows.
+#define LZ_RUN_BLOCKS 4096
+extern "C" int qs_lanczos_run_ctl_bytes() { return (int)sizeof(LzRunCtl); }
+extern "C" int64_t qs_lanczos_run_scratch_doubles(int m, int reorth)
+{
+    return LZ_RUN_BLOCKS + 2 + (reorth ? qs_lanczos_reorth_scratch_doubles(m) : 0);
+}
+
+// A whole m-step Lanczos run on a float-pair CSR operand with the vectors kept:
+// Q [m, n] rows, Q[0] the normalised start vector; per step the scaling with
+// the pair split, the product with -b v and the dot product, and the axpy with
+// the norm are one launch each (the separate calls above take nine: scale,
+// three for the product, two for alpha, two for beta, and a norm reset).
+// reorth: classical Gram-Schmidt against all earlier rows, a second pass when
+// the first lost more than 1 - 1/sqrt(2) of the norm, decided on the device.
+// pdtype: plain pairs (QS_PF / QS_CPF) or packed codes (QS_PF8P / QS_CPF8P),
+// int32 indptr; group: launch shape of the product.  r: n elements; xs: n split
+// elements (8 or 16 bytes each); ab: a[m], b[m]; ctl: qs_lanczos_run_ctl_bytes
+// of zeros with m_eff (the second word) set to m.
+extern "C" int qs_lanczos_run(int64_t n, int m, int cplx, double eps, int reorth, const int32_t *indptr,
+                              const int32_t *indices, const void *pdata, int pdtype, int group, double *Q, double *r,
+                              void *xs, double *ab, double *scratch, void *ctl, void *stream)
+{
+    if (n < 1 || m < 1 || !indptr || !indices || !pdata || !Q || !r || !xs || !ab || !scratch || !ctl)
+        return QS_ERR_ARG;
+    cudaStream_t st = qs_stream(stream);
+    LzRunCtl *c = (LzRunCtl *)ctl;
+    const LzCtl *c1 = (const LzCtl *)ctl;
+    const int64_t n2 = cplx ? 2 * n : n;
+    // the vector passes end in a sum over blocks: two blocks per SM keep the
+    // memory system busy and halve the partials of lz_blocks
+    const int nb = lz_blocks(n), two = 2 * qs_num_sms(), nb2 = lz_blocks(n2) < two ? lz_blocks(n2) : two;
+    double *a = ab, *b = ab + m, *partial = scratch, *state = scratch + LZ_RUN_BLOCKS, *part = state + 2;
+    double *h = part + (int64_t)2 * LZ_BLOCKS_MAX * m;
+    int xexp = 0;                                  // 2^xexp >= sqrt(n2)
+    while (((int64_t)1 << (2 * xexp)) < n2) xexp++;
+    for (int i = 0; i < m; i++) {
+        double *q = Q + (int64_t)i * n2;
+        const double *v = i ? q - n2 : nullptr;
+        lz_scale_split_kernel<<<nb2, LZ_THREADS, 0, st>>>(n2, r, i ? b + i - 1 : nullptr, q, (float2 *)xs, xexp,
+                                                         c);
+        const LzProduct p{n, indptr, indices, pdata, xs, xexp, q, v, i ? b + i - 1 : nullptr, r, partial, a + i, c};
+        const int rc = spmv_lanczos(p, pdtype, cplx, group, st);
+        if (rc) return rc;
+        const bool project = reorth && i;
+        lz_axpy_run_kernel<<<nb2, LZ_THREADS, 0, st>>>(n2, r, a + i, q, partial, b + i, project ? LZ_BEFORE : LZ_BETA,
+                                                      eps, i, state, c);
+        for (int pass = 0; project && pass < 2; pass++) {
+            const double *skip = pass ? state + 1 : nullptr;
+            const int nk = i + 1, nacc = cplx ? 2 * nk : nk;
+            if (cplx) lz_gemv_t_kernel<true><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, n2, r, part, c1, skip);
+            else lz_gemv_t_kernel<false><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, n2, r, part, c1, skip);
+            lz_gemv_t_finish<<<(nacc + 7) / 8, 256, 0, st>>>(nb, nk, cplx, part, h, c1, skip);
+            if (cplx)
+                lz_gemv_n_run_kernel<true><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, n2, h, r, partial, b + i, eps, i, state,
+                                                                     pass, c);
+            else
+                lz_gemv_n_run_kernel<false><<<nb, LZ_THREADS, 0, st>>>(n, nk, Q, n2, h, r, partial, b + i, eps, i, state,
+                                                                      pass, c);
+        }
+        QS_CHECK(cudaGetLastError());
+    }
     return QS_OK;
 }
 

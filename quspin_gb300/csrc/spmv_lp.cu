@@ -20,6 +20,7 @@
 #include "qs_common.cuh"
 #include "pairf.cuh"
 #include "lp_lanes.cuh"
+#include "lanczos.cuh"
 
 namespace {
 
@@ -54,12 +55,76 @@ template <class M> __device__ __forceinline__ void st_out(cflt *y, int64_t e, in
     *p = r;
 }
 
+// Sum of one row over its group's G lanes (every lane of the group gets it).
 // VM: 0 one value per nonzero; 1 coded: data holds a table of QS_CODE_TABLE
 // values followed by one code byte per nonzero (pdtype QS_PF8 / QS_CPF8);
 // 2 packed: indices holds col << 8 | code and data the table only (QS_PF8P /
 // QS_CPF8P); 3 packed, one complex vector, the column words read four per
 // 16-byte load (indices readable up to the next multiple of four words).
-// The table is staged in shared memory.
+// tab: the table in shared memory.
+template <class M, class DV, bool XC, class IT, int U, int VM>
+__device__ __forceinline__ void row_sum(const int32_t *__restrict__ indices, const DV *__restrict__ data,
+                                        const uint8_t *__restrict__ codes, const DV *s_tab,
+                                        const void *__restrict__ xv, unsigned long long keep, IT k0, IT k1, int lane,
+                                        int G, typename M::S &ar, typename M::S &ai)
+{
+    using S = typename M::S;
+    using BE = typename M::BE;
+    const BE *xc = reinterpret_cast<const BE *>(xv);
+    const S *xr = reinterpret_cast<const S *>(xv);
+    ar = ai = M::zero();
+    if constexpr (VM == 3) {
+        // the row's packed column words in 16-byte aligned groups of four,
+        // group g of the row to lane g mod G
+        for (IT c = (k0 & ~(IT)3) + 4 * lane; c < k1; c += (IT)(4 * G)) {
+            const uint4 w4 = __ldcs(reinterpret_cast<const uint4 *>(indices + c));
+            const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int h = 0; h < 4; h += 2) {
+                BE bv[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    bv[i] = (c + h + i >= k0 && c + h + i < k1) ? M::ldB(xc + (int32_t)(w[h + i] >> 8), keep)
+                                                                : BE{M::zero(), M::zero()};
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    if (c + h + i >= k0 && c + h + i < k1) vmul_acc<M>(ar, ai, s_tab[w[h + i] & 255u], bv[i]);
+            }
+        }
+    } else {
+        for (IT k = k0 + lane; k < k1; k += (IT)(G * U)) {
+            int32_t col[U];
+            DV d[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const IT kk = k + (IT)(u * G);
+                const bool in = kk < k1;
+                if constexpr (VM == 2) {
+                    const uint32_t w = in ? (uint32_t)__ldcs(indices + kk) : 0u;
+                    col[u] = (int32_t)(w >> 8);
+                    d[u] = in ? s_tab[w & 255u] : vzero<DV>();
+                } else {
+                    col[u] = in ? __ldcs(indices + kk) : 0;
+                    if constexpr (VM == 1) d[u] = in ? s_tab[__ldcs(codes + kk)] : vzero<DV>();
+                    else d[u] = in ? ldv(data + kk) : vzero<DV>();
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (k + (IT)(u * G) < k1) {
+                    if constexpr (XC) vmul_acc<M>(ar, ai, d[u], M::ldB(xc + col[u], keep));
+                    else rmul_acc<M>(ar, ai, d[u], M::ldS(xr + col[u]));
+                }
+            }
+        }
+    }
+    for (int o = G >> 1; o > 0; o >>= 1) {
+        ar = M::merge(ar, M::shfl_xor(ar, o));
+        if constexpr (XC || is_cx<DV>::value) ai = M::merge(ai, M::shfl_xor(ai, o));
+    }
+}
+
+// One vector (VM: see row_sum); the table is staged in shared memory.
 template <class M, class DV, bool XC, class YT, class IT, int U, int VM>
 __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const IT *__restrict__ indptr,
                                                       const int32_t *__restrict__ indices,
@@ -68,7 +133,6 @@ __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const 
                                                       const unsigned long long *__restrict__ xnorm)
 {
     using S = typename M::S;
-    using BE = typename M::BE;
     constexpr bool COUT = XC || is_cx<DV>::value;
     __shared__ S s_a[2];
     __shared__ int s_k;
@@ -86,8 +150,6 @@ __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const 
     const cx<S> av{s_a[0], s_a[1]};
     const int k2 = s_k;
     const unsigned long long keep = l2_keep_policy();
-    const BE *xc = reinterpret_cast<const BE *>(xv);
-    const S *xr = reinterpret_cast<const S *>(xv);
 
     const int G = 1 << lgG;
     const int GPW = 32 >> lgG;
@@ -101,56 +163,8 @@ __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const 
         const bool valid = r < n;
         const bool writer = valid && (COUT ? lane < 2 : lane == 0);
         const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
-        S ar = M::zero(), ai = M::zero();
-        if constexpr (VM == 3) {
-            // the row's packed column words in 16-byte aligned groups of four,
-            // group g of the row to lane g mod G
-            for (IT c = (k0 & ~(IT)3) + 4 * lane; c < k1; c += (IT)(4 * G)) {
-                const uint4 w4 = __ldcs(reinterpret_cast<const uint4 *>(indices + c));
-                const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                for (int h = 0; h < 4; h += 2) {
-                    BE bv[2];
-#pragma unroll
-                    for (int i = 0; i < 2; i++)
-                        bv[i] = (c + h + i >= k0 && c + h + i < k1) ? M::ldB(xc + (int32_t)(w[h + i] >> 8), keep)
-                                                                    : BE{M::zero(), M::zero()};
-#pragma unroll
-                    for (int i = 0; i < 2; i++)
-                        if (c + h + i >= k0 && c + h + i < k1) vmul_acc<M>(ar, ai, s_tab[w[h + i] & 255u], bv[i]);
-                }
-            }
-        } else {
-            for (IT k = k0 + lane; k < k1; k += (IT)(G * U)) {
-                int32_t col[U];
-                DV d[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const IT kk = k + (IT)(u * G);
-                    const bool in = kk < k1;
-                    if constexpr (VM == 2) {
-                        const uint32_t w = in ? (uint32_t)__ldcs(indices + kk) : 0u;
-                        col[u] = (int32_t)(w >> 8);
-                        d[u] = in ? s_tab[w & 255u] : vzero<DV>();
-                    } else {
-                        col[u] = in ? __ldcs(indices + kk) : 0;
-                        if constexpr (VM == 1) d[u] = in ? s_tab[__ldcs(codes + kk)] : vzero<DV>();
-                        else d[u] = in ? ldv(data + kk) : vzero<DV>();
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (k + (IT)(u * G) < k1) {
-                        if constexpr (XC) vmul_acc<M>(ar, ai, d[u], M::ldB(xc + col[u], keep));
-                        else rmul_acc<M>(ar, ai, d[u], M::ldS(xr + col[u]));
-                    }
-                }
-            }
-        }
-        for (int o = G >> 1; o > 0; o >>= 1) {
-            ar = M::merge(ar, M::shfl_xor(ar, o));
-            if constexpr (COUT) ai = M::merge(ai, M::shfl_xor(ai, o));
-        }
+        S ar, ai;
+        row_sum<M, DV, XC, IT, U, VM>(indices, data, codes, s_tab, xv, keep, k0, k1, lane, G, ar, ai);
         if (writer) {
             const S accr = M::fin(ar);
             if constexpr (COUT) {
@@ -163,6 +177,48 @@ __global__ void __launch_bounds__(256) spmv_lp_kernel(int64_t n, int lgG, const 
             }
         }
     }
+}
+
+// The product of a Lanczos step with the rest of its row work: r = A q - b v
+// and the block's share of Re <q, r> (csrc/lanczos.cu: the step; xs: q split
+// into pairs at a fixed scale).  The same row sums as spmv_lp_kernel;
+// the three FP64 instructions per component ride on rows that are otherwise
+// bound by their gathers, and r is written once.
+template <class DV, bool XC, int U, int VM>
+__global__ void __launch_bounds__(256) spmv_lz_kernel(LzProduct p, int lgG)
+{
+    using M = ModePF;
+    constexpr bool CODED = VM != 0;
+    __shared__ DV s_tab[CODED ? QS_CODE_TABLE : 1];
+    if (p.ctl->done) return;
+    const DV *data = reinterpret_cast<const DV *>(p.data);
+    if constexpr (CODED) {
+        for (int i = threadIdx.x; i < QS_CODE_TABLE; i += blockDim.x) s_tab[i] = ldv(data + i);
+        __syncthreads();
+    }
+    const int32_t *__restrict__ indptr = p.indptr;
+    const unsigned long long keep = l2_keep_policy();
+    const double bv = p.v ? *p.b : 0.0;
+    const int G = 1 << lgG, GPW = 32 >> lgG, lane = threadIdx.x & (G - 1), comp = lane & 1;
+    const int gsub = (threadIdx.x & 31) >> lgG;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    double dot = 0.0;
+    for (int64_t rb = warp * GPW; rb < p.n; rb += nwarps * GPW) {
+        const int64_t r = rb + gsub;
+        const bool valid = r < p.n;
+        const int32_t k0 = valid ? indptr[r] : 0, k1 = valid ? indptr[r + 1] : 0;
+        pf ar, ai;
+        row_sum<M, DV, XC, int32_t, U, VM>(p.indices, data, nullptr, s_tab, p.xs, keep, k0, k1, lane, G, ar, ai);
+        if (valid && (XC ? lane < 2 : lane == 0)) {
+            const int64_t e = XC ? 2 * r + comp : r;
+            double rr = M::to_d(M::fin(XC && comp ? ai : ar), -p.xexp);
+            if (p.v) rr = fma(-bv, __ldg(p.v + e), rr);
+            p.r[e] = rr;
+            dot = fma(__ldg(p.q + e), rr, dot);
+        }
+    }
+    lz_block_finish(dot, p.partial, p.alpha, LZ_SUM, 0.0, 0, nullptr, p.ctl);
 }
 
 // Several vectors: the vectors across the lanes (vl_row_sum), VL lanes to a
@@ -364,6 +420,47 @@ int spmv_lp_single(int64_t n, const void *indptr, int idx64, const int32_t *indi
     if (xtype == QS_C64 && dtype == QS_F32) return spmv_idx<ModeF32, float, true, cflt>(s);
     if (xtype == QS_C64 && dtype == QS_C64) return spmv_idx<ModeF32, cx<float>, true, cflt>(s);
     return QS_ERR_UNSUPPORTED;
+}
+
+namespace {
+template <class DV, bool XC, int U, int VM>
+int lz_go(const LzProduct &p, int G, cudaStream_t st)
+{
+    int lg = 0;
+    while ((1 << lg) < G) lg++;
+    static int resident = 0;
+    auto k = spmv_lz_kernel<DV, XC, U, VM>;
+    k<<<qs_persistent_grid(k, 256, grid_rows(p.n, G), resident), 256, 0, st>>>(p, lg);
+    QS_CHECK(cudaGetLastError());
+    return QS_OK;
+}
+template <class DV, bool XC, int VM>
+int lz_u(const LzProduct &p, int G, int U, cudaStream_t st)
+{
+    if (U >= 4) return lz_go<DV, XC, 4, VM>(p, G, st);
+    if (U >= 2) return lz_go<DV, XC, 2, VM>(p, G, st);
+    return lz_go<DV, XC, 1, VM>(p, G, st);
+}
+}  // namespace
+
+// The fused product of a Lanczos step: plain pairs or packed codes (int32
+// row pointers), launch shape `group` as for qs_csr_matvec_pairs.
+int spmv_lanczos(const LzProduct &p, int pdtype, int cplx, int group, cudaStream_t st)
+{
+    int G = group > 0 ? (group & 0xff) : 2, U = group > 0 ? ((group >> 8) & 0xff) : 1;
+    if (G != 2 && G != 4 && G != 8 && G != 16 && G != 32) return QS_ERR_ARG;
+    const bool v4 = group > 0 && ((group >> 20) & 7) == 6;
+    switch (pdtype) {
+    case QS_PF: return cplx ? lz_u<pf, true, 0>(p, G, U, st) : lz_u<pf, false, 0>(p, G, U, st);
+    case QS_CPF: return cplx ? lz_u<cpf, true, 0>(p, G, U, st) : QS_ERR_ARG;
+    case QS_PF8P:
+        if (v4) return cplx ? lz_go<pf, true, 1, 3>(p, G, st) : QS_ERR_ARG;
+        return cplx ? lz_u<pf, true, 2>(p, G, U, st) : lz_u<pf, false, 2>(p, G, U, st);
+    case QS_CPF8P:
+        if (!cplx) return QS_ERR_ARG;
+        return v4 ? lz_go<cpf, true, 1, 3>(p, G, st) : lz_u<cpf, true, 2>(p, G, U, st);
+    default: return QS_ERR_ARG;
+    }
 }
 
 // y = a A x (overwrite) or y += a A x with float64 / complex128 x and y and

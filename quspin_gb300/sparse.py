@@ -111,15 +111,15 @@ class DeviceCSR:
             self._xs = sc
         return sc
 
-    def _spmv_operand(self):
-        """The float-pair operand of the next product: plain pairs for the
+    def _spmv_operand(self, products=1):
+        """The float-pair operand of the next ``products`` products: plain pairs for the
         first CODE_AFTER_PRODUCTS products of a matrix, then the coded form
         (one sort of the values, worth it for a reused matrix; at once when
         a Taylor operand exists), with the codes packed into the column words
         where that applies."""
         P = self.__dict__.get("_paired_coded")
         if P is None:
-            self._nprod = self.__dict__.get("_nprod", 0) + 1
+            self._nprod = self.__dict__.get("_nprod", 0) + products
             P = self.paired(coded=self._nprod > self.CODE_AFTER_PRODUCTS)
         Pk = P.packed() if P.coded else None
         return P if Pk is None else Pk

@@ -79,6 +79,19 @@ class _DeviceOp:
     def __call__(self, x, y):
         self._f(x, y)
 
+    def pair_csr(self, cplx):
+        """The device CSR whose float-pair product is all of this operator on
+        float64 (complex128 when cplx) vectors, or None."""
+        from ..operators import hamiltonian
+        from .. import sparse
+        M = self.A
+        if isinstance(M, hamiltonian):
+            M = None if M._dynamic else M._static
+        if (self._x32 is not None or self._f == self._single or not isinstance(M, DeviceCSR) or M.idx64
+                or M.nnz == 0 or sparse.SPMV_PRECISION != "double" or (M.dtype.kind == "c" and not cplx)):
+            return None
+        return M
+
 
 def _work_dtype(dtype):
     return np.dtype(np.complex128) if np.dtype(dtype).kind == "c" else np.dtype(np.float64)
@@ -95,6 +108,25 @@ def _recurrence(op, q0, m, eps, Q=None, reorth=False):
     st = D.stream()
     ab = torch.zeros(2 * m + 1, dtype=torch.float64, device=D.device())
     a_d, b_d = ab[:m], ab[m:2 * m]
+    M = op.pair_csr(cplx) if Q is not None else None
+    P = None if M is None else M._spmv_operand(m)
+    if P is not None and P.vcode not in (_lib.PF8, _lib.CPF8):
+        # a float-pair matrix with the vectors kept: the whole run in one call
+        # (three launches a step).  Everything else takes the step by step loop
+        # below; so does lanczos_iter, whose second pass repeats that loop
+        from ..tune import tune_spmv
+        group = tune_spmv(M, 1, np.complex128 if cplx else np.float64, "double", operand=P)
+        r = torch.empty_like(q0)
+        xs, _ = M._pair_scratch(n2)
+        scr = D.scratch_doubles(L.qs_lanczos_run_scratch_doubles(m, int(reorth)))
+        ctl = torch.zeros(L.qs_lanczos_run_ctl_bytes() // 4, dtype=torch.int32, device=D.device())
+        ctl[1] = m
+        dv = lambda t: D.ptr(torch.view_as_real(t) if t.is_complex() else t)
+        _lib.check(L.qs_lanczos_run(n, m, cplx, float(eps), int(reorth), D.ptr(M.indptr), D.ptr(P.indices),
+                                    D.ptr(P.data), P.vcode, int(group), dv(Q), dv(r), D.ptr(xs), D.ptr(ab),
+                                    D.ptr(scr), D.ptr(ctl), st), "qs_lanczos_run")
+        m_eff = int(ctl[1].item())
+        return D.to_host(a_d), D.to_host(b_d), m_eff, r, ab
     scr = D.scratch_doubles(L.qs_lanczos_scratch_doubles())
     ctl = torch.zeros(2, dtype=torch.int32, device=D.device())
     ctl[1] = m
