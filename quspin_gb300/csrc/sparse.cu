@@ -169,12 +169,17 @@ __global__ void __launch_bounds__(256) csr_spmm_kernel(int64_t n, const IT *__re
 }
 
 // Lanes per row from the mean row length: about 12-24 entries per lane (random
-// gathers favour few lanes per row; the tuner refines this).
+// gathers favour few lanes per row; the tuner refines this).  A matrix of few
+// rows takes more, up to one entry per lane, until some 48 k lanes are at
+// work: with two lanes 4752 rows of 11 entries leave the chip waiting for one
+// load after another (4.8 us; 3.5 us with eight), while at 14.5 k rows and
+// more the reduction's FP64 adds cost what the lanes gain.
 static int pick_group(int64_t n, int64_t nnz)
 {
     double avg = n > 0 ? (double)nnz / (double)n : 1.0;
     int g = 2;
     while (g < 32 && g * 24 < avg) g <<= 1;
+    while (g < 32 && g < avg && 2 * g * n <= 48000) g <<= 1;
     return g;
 }
 

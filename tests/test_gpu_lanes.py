@@ -90,3 +90,23 @@ def test_pairs_without_fp64(cuda):
     fine = ~np.isnan(lo)
     np.testing.assert_array_equal(got[fine, 1], lo[fine])
     assert np.all(np.isnan(got[~fine, 1]))
+
+
+@pytest.mark.parametrize("n", [3, 245, 4752, 30000])
+@pytest.mark.parametrize("k", [1, 2, 5])
+def test_small_products_default_form(cuda, n, k):
+    """The default product of a small matrix is the IEEE form, at every lane
+    count its row count picks, within FP64 rounding of each row; a large one
+    stays in float pairs."""
+    from quspin_gb300 import _device as D
+    from quspin_gb300.sparse import DeviceCSR
+    rng = np.random.default_rng(n + k)
+    A = sp.random(n, n, density=min(1.0, 12.0 / n), random_state=rng, format="csr")
+    x = rng.normal(size=(n, k)) + 1j * rng.normal(size=(n, k))
+    x = x[:, 0].copy() if k == 1 else x
+    M = DeviceCSR.from_scipy(A)
+    assert M._small(k, True) == (2 * M.nnz * k <= (3_000_000 if k <= 2 else 1_000_000))
+    y = M.dot(D.to_device(x))
+    # up to 30 entries a row: at most 64 roundings of 2^-53 in the IEEE form, 48-bit pairs otherwise
+    assert np.all(abs(D.to_host(y) - A @ x) <= (1e-14 if M._small(k, True) else 1e-13) * (abs(A) @ abs(x)))
+    assert ("_paired" in M.__dict__) == (not M._small(k, True))
