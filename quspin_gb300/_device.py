@@ -47,8 +47,13 @@ def require_cuda():
 
 
 def device():
-    require_cuda()
+    if not torch.cuda.is_initialized():
+        require_cuda()
     return torch.device("cuda", torch.cuda.current_device())
+
+
+# element type codes of the C ABI by tensor dtype
+TORCH_CODE = {tt: _NP_TO_CODE[nt] for tt, nt in _TORCH_TO_NP.items() if nt in _NP_TO_CODE}
 
 
 def code(dtype):
@@ -64,7 +69,9 @@ def np_dtype(tdtype):
 
 
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the raw handle: building the Stream object of torch.cuda.current_stream()
+    # costs several microseconds, more than a launch
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def ptr(t):

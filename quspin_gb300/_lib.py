@@ -154,6 +154,7 @@ def check(rc, what):
 
 
 def call(name, *args):
-    rc = getattr(load(), name)(*args)
-    check(rc, name)
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != 0:
+        check(rc, name)
     return rc

@@ -17,6 +17,8 @@ the reference passes them) or CUDA torch tensors (kept on the device).
 """
 from __future__ import annotations
 
+import functools
+
 import numpy as np
 import scipy.sparse as sp
 import torch
@@ -87,6 +89,17 @@ class function:
 
 def _is_opstr_entry(e):
     return isinstance(e, (list, tuple)) and len(e) >= 2 and isinstance(e[0], str)
+
+
+@functools.lru_cache(maxsize=None)
+def _keeps_dtype(tdtype, mdtype, maybe_complex_a):
+    """Whether a product with tensors of this dtype is of the same dtype
+    whatever the scale (a scale of another type than int or float counts as
+    complex)."""
+    if tdtype not in D.TORCH_CODE:
+        return False
+    vdt = D.np_dtype(tdtype)
+    return result_dtype(vdt, mdtype) == vdt and not (maybe_complex_a and vdt.kind != "c")
 
 
 def ishamiltonian(x):
@@ -204,6 +217,15 @@ class hamiltonian:
     # -- products -------------------------------------------------------------
     def dot(self, V, time=0, check=True, out=None, overwrite_out=True, a=1.0):
         """a H(time) V (hamiltonian_core.py:615-788)."""
+        if (out is None and type(V) is torch.Tensor and V.is_cuda and type(time) in (int, float)
+                and V.dim() in (1, 2) and V.is_contiguous() and V.shape[0] == self._shape[1]
+                and _keeps_dtype(V.dtype, self._dtype, type(a) not in (int, float))):
+            # a device vector or block of the result type: nothing to check or convert
+            y = torch.empty_like(V)
+            self._static.matvec_into(V, y, a=a, overwrite=True)
+            for fn, Hd in self._dynamic.items():
+                Hd.matvec_into(V, y, a=a * fn(time), overwrite=False)
+            return y
         if ishamiltonian(V):
             raise NotImplementedError("operator algebra between hamiltonians is not part of the GPU path")
         times = np.array(time)

@@ -146,25 +146,25 @@ class DeviceCSR:
         to use (None: the matrix's current one; the tuner pins it)."""
         n = self.shape[0]
         nvec = 1 if x.dim() == 1 else x.shape[1]
-        xt = D.np_dtype(x.dtype)
+        xcode = D.TORCH_CODE[x.dtype]
+        cplx = xcode in (_lib.C64, _lib.C128)
         prec = SPMV_PRECISION if precision is None else precision
-        paired = (prec == "double" and xt in (np.dtype(np.float64), np.dtype(np.complex128))
-                  and not (self.dtype.kind == "c" and xt.kind != "c"))
-        if paired and precision is None and operand is None and group is None and self._small(nvec, xt.kind == "c"):
+        paired = prec == "double" and xcode in (_lib.F64, _lib.C128) and (cplx or self.dtype.kind != "c")
+        if paired and precision is None and operand is None and group is None and self._small(nvec, cplx):
             paired, group = False, 0
         P = (operand if operand is not None else self._spmv_operand()) if paired else None
         if group is None:
             from .tune import tune_spmv
-            group = tune_spmv(self, nvec, xt, prec, operand=P)
+            group = tune_spmv(self, nvec, D.np_dtype(x.dtype), prec, operand=P)
         a = complex(a)
         if paired:
-            xs, nrm = self._pair_scratch(x.numel() * (2 if xt.kind == "c" else 1))
+            xs, nrm = self._pair_scratch(x.numel() * (2 if cplx else 1))
             _lib.call("qs_csr_matvec_pairs", n, self.nnz, D.ptr(self.indptr), self.idx64, D.ptr(P.indices),
-                      D.ptr(P.data), P.vcode, D.ptr(x), D.code(xt), D.ptr(y), nvec, a.real, a.imag,
+                      D.ptr(P.data), P.vcode, D.ptr(x), xcode, D.ptr(y), nvec, a.real, a.imag,
                       int(bool(overwrite)), int(group), D.ptr(xs), D.ptr(nrm), D.stream())
             return y
         _lib.call("qs_csr_matvec", n, self.nnz, D.ptr(self.indptr), self.idx64, D.ptr(self.indices),
-                  D.ptr(self.data), D.code(self.dtype), D.ptr(x), D.code(xt), D.ptr(y), nvec, a.real, a.imag,
+                  D.ptr(self.data), D.code(self.dtype), D.ptr(x), xcode, D.ptr(y), nvec, a.real, a.imag,
                   int(bool(overwrite)), int(group), D.stream())
         return y
 
@@ -287,7 +287,7 @@ class DeviceDIA:
         nvec = 1 if x.dim() == 1 else x.shape[1]
         a = complex(a)
         _lib.call("qs_dia_matvec", n, int(self.offsets.numel()), D.ptr(self.offsets), int(self.data.shape[1]),
-                  D.ptr(self.data), D.code(self.dtype), D.ptr(x), D.code(D.np_dtype(x.dtype)), D.ptr(y), nvec,
+                  D.ptr(self.data), D.code(self.dtype), D.ptr(x), D.TORCH_CODE[x.dtype], D.ptr(y), nvec,
                   a.real, a.imag, int(bool(overwrite)), D.stream())
         return y
 

@@ -55,15 +55,14 @@ class DeviceDOP853:
         self._e5 = np.ascontiguousarray(self.E5[:self.ns + 1])
         self._e3 = np.ascontiguousarray(self.E3[:self.ns + 1])
         self.rhs = rhs
-        self.y = y0.clone()
+        self.y = y0.clone(memory_format=torch.contiguous_format)
         self.t = float(t0)
         self.rtol, self.atol = float(rtol), float(atol)
         self.nsteps = int(np.iinfo(np.int32).max if nsteps is None else nsteps)
         self.max_step = float(max_step)
         self.h = float(first_step)
         self.shape = y0.shape
-        self._real = self._r(self.y)
-        self.n2 = self._real.numel()
+        self.n2 = self.y.numel() * (2 if self.y.is_complex() else 1)
         dev = y0.device
         self.K = torch.empty((self.ns + 1,) + tuple(self.y.shape), dtype=y0.dtype, device=dev)
         self.ytmp = torch.empty_like(self.y)
@@ -71,38 +70,37 @@ class DeviceDOP853:
         L = _lib.load()
         self._scr = torch.zeros(max(L.qs_rk_error_scratch_doubles(self.n2), 1), dtype=torch.float64, device=dev)
         self._err = torch.zeros(2, dtype=torch.float64, device=dev)
-        self.rhs(self.t, self.y, self.K[0])
+        # per stage: its coefficients as a contiguous row and its row of K
+        self._rows = [np.ascontiguousarray(self.A[s][:s]) for s in range(self.ns)]
+        self.B = np.ascontiguousarray(self.B)
+        self._k = [self.K[s] for s in range(self.ns + 1)]
+        self.rhs(self.t, self.y, self._k[0])
         self.nfev, self.naccept, self.nreject = 1, 0, 0
         self._facold = 1e-4
         self._reject = False
 
-    @staticmethod
-    def _r(x):
-        return torch.view_as_real(x).reshape(-1) if x.is_complex() else x.reshape(-1)
-
-    def _combine(self, coef, nk, h, out):
-        c = np.ascontiguousarray(coef[:nk], np.float64)
-        _lib.call("qs_rk_combine", self.n2, D.ptr(self._r(self.y)), D.ptr(self.K), nk,
-                  c.ctypes.data, h, D.ptr(self._r(out)), D.stream())
+    def _combine(self, c, nk, h, out):
+        """out = y + h sum_j c[j] K[j] (c: contiguous float64)."""
+        _lib.call("qs_rk_combine", self.n2, D.ptr(self.y), D.ptr(self.K), nk, c.ctypes.data, h, D.ptr(out), D.stream())
 
     def _sumsq(self, K, coef, nk):
         """sum_i ((sum_j coef_j K_j)_i / sk_i)^2 with sk = atol + rtol |y_i|
         (one pass of the error kernel with y as both end points)."""
         c = np.zeros(nk, np.float64)
         c[:] = coef
-        y = D.ptr(self._r(self.y))
+        y = D.ptr(self.y)
         _lib.call("qs_rk_error", self.n2, y, y, D.ptr(K), nk, c.ctypes.data, c.ctypes.data, self.atol, self.rtol,
                   D.ptr(self._scr), D.ptr(self._err), D.stream())
         return float(self._err[0].item())
 
     def _initial_step(self, hmax, direction):
         """Hairer's starting-step heuristic (HNW I, II.4) on the scaled norms."""
-        dnf = self._sumsq(self.K[0], [1.0], 1)
+        dnf = self._sumsq(self._k[0], [1.0], 1)
         dny = self._sumsq(self.y, [1.0], 1)
         h = 1e-6 if (dnf <= 1e-10 or dny <= 1e-10) else 0.01 * np.sqrt(dny / dnf)
         h = min(h, hmax) * direction
         self._combine(np.array([1.0]), 1, h, self.ytmp)          # y + h f0
-        self.rhs(self.t + h, self.ytmp, self.K[1])
+        self.rhs(self.t + h, self.ytmp, self._k[1])
         self.nfev += 1
         der2 = np.sqrt(self._sumsq(self.K, [-1.0, 1.0], 2)) / abs(h)
         der12 = max(abs(der2), np.sqrt(dnf))
@@ -133,12 +131,12 @@ class DeviceDOP853:
                 last = True
             steps += 1
             for s in range(1, self.ns):
-                self._combine(self.A[s], s, h, self.ytmp)
-                self.rhs(self.t + self.C[s] * h, self.ytmp, self.K[s])
+                self._combine(self._rows[s], s, h, self.ytmp)
+                self.rhs(self.t + self.C[s] * h, self.ytmp, self._k[s])
             self._combine(self.B, self.ns, h, self.ynew)
-            self.rhs(self.t + h, self.ynew, self.K[self.ns])
+            self.rhs(self.t + h, self.ynew, self._k[self.ns])
             self.nfev += self.ns
-            _lib.call("qs_rk_error", self.n2, D.ptr(self._r(self.y)), D.ptr(self._r(self.ynew)), D.ptr(self.K),
+            _lib.call("qs_rk_error", self.n2, D.ptr(self.y), D.ptr(self.ynew), D.ptr(self.K),
                       self.ns + 1, self._e5.ctypes.data, self._e3.ctypes.data, self.atol, self.rtol,
                       D.ptr(self._scr), D.ptr(self._err), D.stream())
             e5, e3 = self._err.tolist()
@@ -157,7 +155,7 @@ class DeviceDOP853:
                 self.naccept += 1
                 self.t += h
                 self.y, self.ynew = self.ynew, self.y
-                self.K[0].copy_(self.K[self.ns])
+                self._k[0].copy_(self._k[self.ns])
                 if abs(hnew) > hmax:
                     hnew = direction * hmax
                 if self._reject:
@@ -238,8 +236,12 @@ def evolve_hamiltonian(H, v0, t0, times, eom="SE", solver_name="dop853", stack_s
     y0 = D.to_device(v0a, dt).clone() if host else v0a.to(D.torch_dtype(dt)).clone()
     norm0 = torch.linalg.vector_norm(y0, dim=0)
 
+    parts = [(None, H._static)] + list(H._dynamic.items())
+
     def rhs(t, y, out):
-        H.dot(y, time=t, out=out, a=a)
+        # H.dot(y, time=t, out=out, a=a) for vectors of the right type
+        for fn, M in parts:
+            M.matvec_into(y, out, a=a if fn is None else a * fn(t), overwrite=fn is None)
 
     rtol = solver_args.pop("rtol", None)
     atol = solver_args.pop("atol", None)
