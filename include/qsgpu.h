@@ -185,6 +185,15 @@ int qs_expm_multiply(int64_t n, int64_t nnz, const void *d_indptr, int idx64, co
                      const void *d_data, int dtype, void *d_F, int64_t nvec, int s, int m_star, double tol,
                      double mu_re, double mu_im, const void *d_coeff, const void *d_eta, const void *d_one,
                      void *d_work, int btype, void *d_ctl, int group, void *stream);
+/* The same for one vector in float-pair storage on a small int32 matrix (at
+ * most 2^17 rows; dtype 4 / 5, or coded 6 / 7) as one cooperative launch.
+ * d_sync: qs_expm_small_sync_bytes() of zeros before the first call; calls
+ * that share d_work, d_ctl or d_sync must not overlap. */
+int qs_expm_small_sync_bytes(void);
+int qs_expm_multiply_small(int64_t n, int64_t nnz, const int32_t *d_indptr, const int32_t *d_indices,
+                           const void *d_data, int dtype, void *d_F, int s, int m_star, double tol, double mu_re,
+                           double mu_im, const void *d_coeff, const void *d_eta, void *d_work, void *d_ctl,
+                           void *d_sync, void *stream);
 /* The same two calls with a row-sum scratch d_rownorm of n double pairs (16n bytes): with bit 16 of group set and
  * more than 8 right-hand sides, the float forms sweep the rows once per chunk of 8 vectors, so the gathered
  * slice of B stays in L2 (the many-state evolutions of hamiltonian_core.py:1472-1486 and block_tools.py:618-795

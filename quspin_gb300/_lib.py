@@ -72,6 +72,9 @@ _SIGS = {
     "qs_nrm2": (_i, [_i64, _vp, _vp, _vp, _vp]),
     "qs_csr_trace": (_i, [_i64, _vp, _i, _vp, _vp, _i, _vp, _vp, _vp]),
     "qs_csr_1_norm": (_i, [_i64, _vp, _i, _vp, _vp, _i, _d, _d, _vp, _vp, _vp, _vp]),
+    "qs_expm_small_sync_bytes": (_i, []),
+    "qs_expm_multiply_small": (_i, [_i64, _i64, _vp, _vp, _vp, _i, _vp, _i, _i, _d, _d, _d, _vp, _vp, _vp, _vp, _vp,
+                                    _vp]),
     "qs_expm_ctl_bytes": (_i, []),
     "qs_split_pairs": (_i, [_i64, _vp, _vp, _vp]),
     "qs_split_pairs_trunc": (_i, [_i64, _vp, _i, _vp, _vp]),

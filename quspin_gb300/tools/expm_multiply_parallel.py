@@ -285,6 +285,9 @@ class ExpmMultiplyParallel:
         n = self._Ad.shape[0]
         nvec = 1 if F.dim() == 1 else F.shape[1]
         tol = float(self._tol if tol is None else tol)
+        if nvec == 1 and F.is_contiguous() and self._small_operand() is not None \
+                and not torch.cuda.is_current_stream_capturing():
+            return self._run_small(F, tol)
         if (work is None and n * nvec <= self.GRAPH_MAX_ELEMS and F.is_contiguous()
                 and not torch.cuda.is_current_stream_capturing()):
             return self._run_graph(F, tol)
@@ -293,6 +296,43 @@ class ExpmMultiplyParallel:
         if work is not None and btype != _lib.C64:
             wbuf = work          # 16-byte elements: the caller's complex128 work array holds both B buffers
         self._consts = self._launch(F, tol, wbuf, ctl)     # kept alive until the stream reaches it
+        self._last_ctl = ctl
+        return F
+
+    # largest problem evolved in one cooperative launch (csrc/expm_small.cu):
+    # below the sizes whose launch shapes are tuned.  Against the graph of one
+    # launch per term: 137 against 274 us at 245 rows, 285 against 661 at 4752,
+    # 1828 against 2262 at 52377
+    SMALL_MAX_ROWS = 65535
+
+    def _small_operand(self):
+        """The coded or plain float-pair operand of the one-launch evolution,
+        or None where it does not apply (other precisions, larger or int64
+        matrices, a launch shape set by hand)."""
+        A = self._Ad
+        if self._precision != "double" or A.idx64 or not 0 < A.shape[0] <= self.SMALL_MAX_ROWS:
+            return None
+        from ..tune import tune_taylor
+        P, btype = self._operand(1)
+        return P if tune_taylor(P, 1, btype) == 0 else None
+
+    def _run_small(self, F, tol):
+        P = self._small_operand()
+        n = self._Ad.shape[0]
+        work, ctl = self._buffers(n, 1, _lib.CPF)
+        sync = self.__dict__.get("_sync")
+        if sync is None:
+            sync = self._sync = torch.zeros(_lib.load().qs_expm_small_sync_bytes() // 8, dtype=torch.int64,
+                                            device=D.device())
+        key = (complex(self._a), complex(self._mu), int(self._s), int(self._m_star))
+        kept = self.__dict__.get("_small_consts")
+        if kept is None or kept[0] != key:
+            kept = self._small_consts = (key, self._const_table())
+        consts, m = kept[1], max(int(self._m_star), 1)
+        mu = complex(self._mu)
+        _lib.call("qs_expm_multiply_small", n, P.nnz, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(P.data), P.vcode,
+                  D.ptr(F), int(self._s), int(self._m_star), tol, mu.real, mu.imag, D.ptr(consts),
+                  D.ptr(consts[m:m + 1]), D.ptr(work), D.ptr(ctl), D.ptr(sync), D.stream())
         self._last_ctl = ctl
         return F
 

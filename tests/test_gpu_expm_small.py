@@ -1,0 +1,91 @@
+"""The one-launch evolution of small problems (csrc/expm_small.cu) against the
+launch per term on the same operand: sizes around a block's and a sweep's rows,
+real and complex, coded and plain values, one and several substeps, a
+substep that runs out of terms, a zero matrix and repeated calls on the same
+scratch; and against scipy.
+
+Tolerance: the same float-pair arithmetic with the row sums split over another
+number of lanes: 48-bit rounding, at most a few hundred terms."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+from scipy.sparse.linalg import expm_multiply
+
+pytestmark = pytest.mark.gpu
+
+
+def _hermitian(n, cplx, coded, rng):
+    A = sp.random(n, n, density=min(1.0, 6.0 / n), random_state=rng, format="csr")
+    A.data = rng.choice(np.array([0.5, -1.0, 0.25]), A.nnz) if coded else rng.normal(size=A.nnz)
+    if cplx:
+        A = A.astype(complex)
+        A.data = A.data * rng.choice(np.array([1.0, 1j]), A.nnz)
+    A = sp.csr_matrix(A + A.conj().T + sp.diags(rng.choice(np.array([-0.5, 1.0]), n)))
+    A.sum_duplicates()
+    return A
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 255, 4751, 19457, 65535])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("coded", [False, True])
+def test_small_matches_launch_per_term(cuda, n, cplx, coded):
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    rng = np.random.default_rng(n + 2 * cplx + coded)
+    A = _hermitian(n, cplx, coded, rng)
+    v = rng.normal(size=n) + 1j * rng.normal(size=n)
+    scale = 10.0 ** rng.integers(-200, 200)
+    u = v / np.linalg.norm(v)
+    v = u * scale
+    for t in (0.02, 1.7):
+        op = ExpmMultiplyParallel(A, a=-1j * t)
+        assert op._small_operand() is not None and op._small_operand().coded == (coded or n <= 31)
+        one = D.to_host(op.dot(D.to_device(v)))
+        terms, missed = op.terms_executed, op.nonconverged_substeps
+        np.testing.assert_array_equal(one, D.to_host(op.dot(D.to_device(v))))       # the scratch is left as it was
+        ExpmMultiplyParallel.SMALL_MAX_ROWS, old = 0, ExpmMultiplyParallel.SMALL_MAX_ROWS
+        try:
+            ref = D.to_host(op.dot(D.to_device(v)))
+        finally:
+            ExpmMultiplyParallel.SMALL_MAX_ROWS = old
+        one, ref = one / scale, ref / scale                    # norms of 1e200 overflow when squared
+        assert np.linalg.norm(one - ref) <= 1e-13 * np.linalg.norm(ref)
+        assert abs(terms - op.terms_executed) <= op.s and missed == op.nonconverged_substeps
+        if n <= 4751:
+            exact = expm_multiply(-1j * t * A, u)
+            assert np.linalg.norm(one - exact) <= 1e-12 * np.linalg.norm(exact)
+
+
+def test_small_edges(cuda):
+    """A substep cut off after three terms is counted; m* = 0 and a zero
+    matrix leave the state; a NaN stays a NaN and the next call is clean."""
+    from quspin_gb300 import _device as D
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    rng = np.random.default_rng(1)
+    n = 1000
+    A = _hermitian(n, False, True, rng)
+    v = rng.normal(size=n) + 1j * rng.normal(size=n)
+    op = ExpmMultiplyParallel(A, a=-1j)
+    full = op.dot(v)
+    op.set_partition(3, 4)
+    cut = op.dot(v)
+    assert op.nonconverged_substeps == 4 and op.terms_executed == 12
+    B, F = None, v.copy()
+    mu = A.diagonal().mean()
+    for _ in range(4):
+        B = F
+        for j in range(3):
+            B = -1j / (4 * (j + 1)) * (A @ B - mu * B)
+            F = F + B if j else F + B
+        F = F * np.exp(-1j * mu / 4)
+    assert np.linalg.norm(cut - F) <= 1e-12 * np.linalg.norm(F)
+    w = v.copy()
+    w[3] = np.nan
+    assert np.isnan(op.dot(w)).any()
+    op._calculate_partition()
+    np.testing.assert_array_equal(op.dot(v), full)
+    Z = ExpmMultiplyParallel(sp.csr_matrix((n, n)), a=-1j)
+    assert Z.m_star == 0
+    np.testing.assert_allclose(Z.dot(v), v, rtol=0, atol=0)
+    assert D.to_device(v).shape == (n,)
