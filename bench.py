@@ -84,6 +84,8 @@ def peak_hbm():
 KERNEL_SOURCES = {
     "taylor_r32_kernel": ["expm_st.cu", "lp_modes.cuh", "pairf.cuh", "expm_ctl.cuh", "qs_common.cuh"],
     "taylor_rows_kernel": ["expm_st.cu", "lp_modes.cuh", "pairf.cuh", "expm_ctl.cuh", "qs_common.cuh"],
+    "taylor_sell_kernel": ["sell.cu", "sell.cuh", "lp_lanes.cuh", "lp_modes.cuh", "pairf.cuh", "expm_ctl.cuh",
+                           "qs_common.cuh"],
     "taylor_lp_kernel": ["expm_lp.cu", "lp_modes.cuh", "pairf.cuh", "expm_ctl.cuh", "qs_common.cuh"],
 }
 
@@ -108,11 +110,14 @@ def profile_traffic(kernel):
     p = os.path.join(ROOT, "profiles", "taylor_term_j1j2.md")
     if not os.path.exists(p):
         return None, "no ncu summary"
-    rec = {}
+    recs = []
     for line in open(p):
         for key in ("traffic_kernel", "traffic_source_sha256", "traffic_bytes_per_launch_full"):
             if line.strip().startswith(key + ":"):
-                rec[key] = line.split(":", 1)[1].strip()
+                if key == "traffic_kernel" or not recs:
+                    recs.append({})
+                recs[-1][key] = line.split(":", 1)[1].strip()
+    rec = next((r for r in recs if r.get("traffic_kernel") == kernel), recs[0] if recs else {})
     if rec.get("traffic_kernel") != kernel:
         return None, "the ncu summary covers {}, not {}".format(rec.get("traffic_kernel"), kernel)
     if rec.get("traffic_source_sha256") != kernel_source_sha(kernel):
@@ -216,6 +221,8 @@ def build_problem(L, J1, J2):
 def taylor_kernel_name(group):
     """Kernel the launch code selects for one vector in the float forms."""
     shape = (group >> 20) & 7
+    if (group >> 23) & 1:
+        return "taylor_sell_kernel"
     return "taylor_rows_kernel" if shape >= 4 else ("taylor_r32_kernel" if shape else "taylor_lp_kernel")
 
 
@@ -717,7 +724,8 @@ def run_ours(args, rank, ws):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind, "traffic": traffic, "traffic_source": traffic_note, "kernel": taylor_kernel_name(group),
                      "algorithmic_bytes_per_launch": tb, "launch_ms": 1e3 * t_term,
-                     "launch_shape": {"lanes_per_row": group & 0xff, "entries_in_flight": (group >> 8) & 0xff,
+                     "launch_shape": {"form": "slices of 32 rows, one row per lane"} if (group >> 23) & 1 else
+                                     {"lanes_per_row": group & 0xff, "entries_in_flight": (group >> 8) & 0xff,
                                       "blocks_per_sm_cap": ({0: 4, 1: 6, 2: 5} if (group >> 20) & 7 else
                                                             {0: None, 1: 6, 2: 8}).get((group >> 18) & 3),
                                       "column_words_per_load": 4 if (group >> 20) & 7 in (6, 7) else 1},
@@ -1076,7 +1084,8 @@ def run_spmv(args):
         nb = spmv_bytes(n, nnz, vb=vb)
         res[prec] = {"ms": 1e3 * t, "algorithmic_bytes": nb, "value_bytes_per_nonzero": vb, "gbs": nb / t / 1e9,
                      "frac_of_hbm_peak": nb / t / 1e9 / peak, "y_checksum": complex(y.sum().item()),
-                     "launch_shape": {"lanes_per_row": code & 0xff, "entries_in_flight": (code >> 8) & 0xff,
+                     "launch_shape": {"form": "slices of 32 rows, one row per lane"} if (code >> 23) & 1 else
+                                     {"lanes_per_row": code & 0xff, "entries_in_flight": (code >> 8) & 0xff,
                                       "column_words_per_load": 4 if (code >> 20) & 7 == 6 else 1}}
     ref = res["ieee"]["y_checksum"]
     out = {"workload": "j1j2_chain_L{}_spmv".format(L), "Ns": n, "nnz": nnz, "build_s": t_build,

@@ -185,6 +185,14 @@ int qs_expm_multiply(int64_t n, int64_t nnz, const void *d_indptr, int idx64, co
                      const void *d_data, int dtype, void *d_F, int64_t nvec, int s, int m_star, double tol,
                      double mu_re, double mu_im, const void *d_coeff, const void *d_eta, const void *d_one,
                      void *d_work, int btype, void *d_ctl, int group, void *stream);
+/* The sliced form of a packed coded matrix (types 10 / 11: one vector, 32 rows
+ * per slice, slots in groups of four) for qs_csr_matvec_pairs, qs_taylor_term,
+ * qs_expm_multiply and qs_lanczos_run; its slice pointers (int64, groups before
+ * each slice) take the place of d_indptr.  Count, scan the groups, then fill
+ * (rows of at most 128 nonzeros; 128 words per group). */
+int qs_sell_count(int64_t n, const int32_t *d_indptr, int64_t *d_groups, int *d_most, void *stream);
+int qs_sell_fill(int64_t n, const int32_t *d_indptr, const int32_t *d_words, const int64_t *d_sptr, int64_t groups,
+                 int32_t *d_out, void *stream);
 /* The same for one vector in float-pair storage on a small int32 matrix (at
  * most 2^17 rows; dtype 4 / 5, or coded 6 / 7) as one cooperative launch.
  * d_sync: qs_expm_small_sync_bytes() of zeros before the first call; calls

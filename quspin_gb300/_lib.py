@@ -18,7 +18,7 @@ _lib = None
 _lock = threading.Lock()
 
 # element type codes shared with the C side
-F32, F64, C64, C128, PF, CPF, PF8, CPF8, PF8P, CPF8P = 0, 1, 2, 3, 4, 5, 6, 7, 8, 9
+F32, F64, C64, C128, PF, CPF, PF8, CPF8, PF8P, CPF8P, PF8S, CPF8S = range(12)
 
 STATUS = {
     -1: "invalid argument",
@@ -73,6 +73,8 @@ _SIGS = {
     "qs_csr_trace": (_i, [_i64, _vp, _i, _vp, _vp, _i, _vp, _vp, _vp]),
     "qs_csr_1_norm": (_i, [_i64, _vp, _i, _vp, _vp, _i, _d, _d, _vp, _vp, _vp, _vp]),
     "qs_expm_small_sync_bytes": (_i, []),
+    "qs_sell_count": (_i, [_i64, _vp, _vp, _vp, _vp]),
+    "qs_sell_fill": (_i, [_i64, _vp, _vp, _vp, _i64, _vp, _vp]),
     "qs_expm_multiply_small": (_i, [_i64, _i64, _vp, _vp, _vp, _i, _vp, _i, _i, _d, _d, _d, _vp, _vp, _vp, _vp, _vp,
                                     _vp]),
     "qs_expm_ctl_bytes": (_i, []),

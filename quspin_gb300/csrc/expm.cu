@@ -25,6 +25,7 @@
 // paired-single and complex64 forms of the same term, selected by btype.
 #include "qs_common.cuh"
 #include "expm_ctl.cuh"
+#include "sell.cuh"
 
 extern "C" int qs_expm_ctl_bytes() { return (int)sizeof(ExpmCtl); }
 extern "C" int qs_multi_ctl_bytes() { return (int)sizeof(MultiCtl); }
@@ -343,6 +344,7 @@ extern "C" int qs_taylor_term_rows(int64_t n, int64_t nnz, const void *indptr, i
         a.nnz = nnz;
         // several vectors without a given shape: the vectors across the lanes
         a.staged = group > 0 ? (group >> 20) & 7 : (nvec > 1 ? 1 : 0);
+        if (sell_type(dtype)) return sell_taylor_term(a);
         if (a.staged) return a.nvec == 1 ? st_taylor_term(a) : vl_taylor_term(a, false);
         return lp_taylor_term(a, false);
     }

@@ -21,6 +21,7 @@
 #include "pairf.cuh"
 #include "lp_lanes.cuh"
 #include "lanczos.cuh"
+#include "sell.cuh"
 
 namespace {
 
@@ -447,6 +448,7 @@ int lz_u(const LzProduct &p, int G, int U, cudaStream_t st)
 // row pointers), launch shape `group` as for qs_csr_matvec_pairs.
 int spmv_lanczos(const LzProduct &p, int pdtype, int cplx, int group, cudaStream_t st)
 {
+    if (sell_type(pdtype)) return sell_lanczos(p, pdtype, cplx, st);
     int G = group > 0 ? (group & 0xff) : 2, U = group > 0 ? ((group >> 8) & 0xff) : 1;
     if (G != 2 && G != 4 && G != 8 && G != 16 && G != 32) return QS_ERR_ARG;
     const bool v4 = group > 0 && ((group >> 20) & 7) == 6;
@@ -469,7 +471,9 @@ int spmv_lanczos(const LzProduct &p, int pdtype, int cplx, int group, cudaStream
 // one code byte per nonzero into a table of such pairs (QS_PF8 / QS_CPF8:
 // QS_CODE_TABLE pairs, then nnz uint8 codes; int32 indices), or with the
 // code packed into the low 8 bits of each column word (QS_PF8P / QS_CPF8P:
-// indices holds col << 8 | code, col < 2^23; pdata the table only).
+// indices holds col << 8 | code, col < 2^23; pdata the table only), or such
+// words in slices of 32 rows (QS_PF8S / QS_CPF8S, one vector: csrc/sell.cu;
+// indptr holds the slice pointers, int64).
 // xs: scratch of n*nvec*(8 or 16) bytes for the split x; norm: 8 bytes of
 // device scratch.  group as for qs_csr_matvec.
 extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, int idx64, const int32_t *indices,
@@ -481,11 +485,12 @@ extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, i
     if (n == 0) return QS_OK;
     const bool xc = xtype == QS_C128;
     if (!xc && xtype != QS_F64) return QS_ERR_ARG;
-    const bool cvals = pdtype == QS_CPF || pdtype == QS_CPF8 || pdtype == QS_CPF8P;
+    const bool cvals = pdtype == QS_CPF || pdtype == QS_CPF8 || pdtype == QS_CPF8P || pdtype == QS_CPF8S;
     if (!xc && (a_im != 0.0 || cvals)) return QS_ERR_ARG;
     if (pdtype != QS_PF && pdtype != QS_CPF && pdtype != QS_PF8 && pdtype != QS_CPF8 && pdtype != QS_PF8P &&
-        pdtype != QS_CPF8P)
+        pdtype != QS_CPF8P && !sell_type(pdtype))
         return QS_ERR_ARG;
+    if (sell_type(pdtype) && nvec != 1) return QS_ERR_ARG;
     if (pdtype != QS_PF && pdtype != QS_CPF && idx64) return QS_ERR_ARG;
     int G = group > 0 ? (group & 0xff) : 2;
     int U = group > 0 ? ((group >> 8) & 0xff) : 1;
@@ -502,6 +507,9 @@ extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, i
     xnorm_kernel<<<nblk, 256, 0, st>>>(count, (const double *)x, nrm);
     xsplit_kernel<<<blocks, 256, 0, st>>>(count, (const double *)x, (float2 *)xs, nrm);
     QS_CHECK(cudaGetLastError());
+    if (sell_type(pdtype))
+        return sell_spmv(n, (const int64_t *)indptr, indices, pdata, pdtype, xs, xc, y, cdbl{a_re, a_im}, overwrite, nrm,
+                         st);
     SpmvArgs s{n, indptr, idx64, indices, pdata, xs, y, nvec, cdbl{a_re, a_im}, overwrite, nrm, G, U, st};
     if (pdtype == QS_PF8) return xc ? spmv_idx<ModePF, pf, true, cdbl, 1>(s) : spmv_idx<ModePF, pf, false, double, 1>(s);
     if (pdtype == QS_CPF8) return spmv_idx<ModePF, cpf, true, cdbl, 1>(s);

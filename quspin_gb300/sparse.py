@@ -25,6 +25,8 @@ from . import _lib
 # complex64 vectors always use FP32 products.
 SPMV_PRECISION = "double"
 
+SLICED = 1 << 23      # launch code bit: the sliced form of a packed operand
+
 # With "double" as the default, products of few enough FP64 multiply-adds take
 # the IEEE form all the same: it is one launch, the pair form four (norm reset,
 # norm, split, product), and no less precise.  Measured on GB300, one vector:
@@ -157,9 +159,13 @@ class DeviceCSR:
             from .tune import tune_spmv
             group = tune_spmv(self, nvec, D.np_dtype(x.dtype), prec, operand=P)
         a = complex(a)
+        indptr = self.indptr
+        if paired and nvec == 1 and group & SLICED:
+            P = P.sliced()
+            indptr = P.indptr
         if paired:
             xs, nrm = self._pair_scratch(x.numel() * (2 if cplx else 1))
-            _lib.call("qs_csr_matvec_pairs", n, self.nnz, D.ptr(self.indptr), self.idx64, D.ptr(P.indices),
+            _lib.call("qs_csr_matvec_pairs", n, self.nnz, D.ptr(indptr), self.idx64, D.ptr(P.indices),
                       D.ptr(P.data), P.vcode, D.ptr(x), xcode, D.ptr(y), nvec, a.real, a.imag,
                       int(bool(overwrite)), int(group), D.ptr(xs), D.ptr(nrm), D.stream())
             return y
@@ -447,6 +453,14 @@ class PackedCodedCSR:
         self.data = P.data[:tbytes].clone()
         self.coded = True
 
+    def sliced(self):
+        """The SlicedCSR form of this operand (cached), or None when it does
+        not apply (a row of more than 128 nonzeros, or rows so uneven that
+        the slices would hold half as much again)."""
+        if "_sliced" not in self.__dict__:
+            self._sliced = SlicedCSR.build(self)
+        return self._sliced
+
     @property
     def nnz(self):
         return self._nnz
@@ -454,6 +468,55 @@ class PackedCodedCSR:
     @property
     def vcode(self):
         return _lib.CPF8P if self.complex else _lib.PF8P
+
+    @property
+    def value_bytes(self):
+        """Bytes of value stream per nonzero beyond the 4-byte column word."""
+        return 0
+
+
+class SlicedCSR:
+    """A PackedCodedCSR in slices of 32 rows for the single-vector kernels of
+    csrc/sell.cu (type codes PF8S / CPF8S): one row per lane, the rows' words in
+    an order that lets the 32 lanes of a warp read common lines of the vector.
+    ``indptr`` holds the slice pointers, in groups of four slots (128 words)."""
+
+    format = "csr"
+    MAX_ROW = 128
+    MAX_PADDING = 1.5
+
+    @classmethod
+    def build(cls, P):
+        n, nnz = P.shape[0], P.nnz
+        if n == 0 or nnz == 0:
+            return None
+        slices = (n + 31) // 32
+        sptr = torch.zeros(slices + 1, dtype=torch.int64, device=D.device())
+        most = torch.zeros(1, dtype=torch.int32, device=D.device())
+        _lib.call("qs_sell_count", n, D.ptr(P.indptr), D.ptr(sptr[1:]), D.ptr(most), D.stream())
+        scr = torch.empty(max(_lib.load().qs_scan_scratch_elems(slices), 1), dtype=torch.int64, device=D.device())
+        _lib.call("qs_scan_inclusive_i64", D.ptr(sptr[1:]), slices, D.ptr(scr), D.stream())
+        groups = int(sptr[-1].item())
+        if int(most.item()) > cls.MAX_ROW or groups * 128 > cls.MAX_PADDING * nnz + 4096:
+            return None
+        S = cls()
+        S.indptr, S.data, S.shape, S.idx64 = sptr, P.data, P.shape, 0
+        S._nnz, S.complex, S.dtype, S.distinct, S.coded = nnz, P.complex, P.dtype, P.distinct, True
+        try:
+            S.indices = torch.empty(groups * 128, dtype=torch.int32, device=D.device())
+        except torch.OutOfMemoryError:      # the packed form serves as well
+            return None
+        _lib.call("qs_sell_fill", n, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(sptr), groups, D.ptr(S.indices),
+                  D.stream())
+        return S
+
+    @property
+    def nnz(self):
+        return self._nnz
+
+    @property
+    def vcode(self):
+        return _lib.CPF8S if self.complex else _lib.PF8S
 
     @property
     def value_bytes(self):

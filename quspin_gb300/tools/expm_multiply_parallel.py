@@ -215,9 +215,9 @@ class ExpmMultiplyParallel:
 
     def _operand(self, nvec=1):
         """(matrix in the value form of the precision, B storage code).  For
-        one vector in the float-pair form, the coded operand and its packed
-        form (code bytes inside the column words) are both tuned once and the
-        faster is kept."""
+        one vector in the float-pair form, the coded operand, its packed form
+        (code bytes inside the column words) and that in slices are tuned once
+        and the fastest is kept."""
         if self._precision == "mixed":
             return self._mixed_matrix(), _lib.C64
         if self._precision == "ieee":
@@ -231,13 +231,14 @@ class ExpmMultiplyParallel:
             Pk = P.packed() if P.shape[0] >= 65536 else None
             if Pk is not None:
                 from ..tune import tune_taylor
-                tune_taylor(P, 1, _lib.CPF)
-                tune_taylor(Pk, 1, _lib.CPF)
-                key = ("taylor", 1, _lib.CPF)
-                t_plain = P.__dict__.get("_tuned_ms", {}).get(key)
-                t_pack = Pk.__dict__.get("_tuned_ms", {}).get(key)
-                if t_pack is not None and t_plain is not None and t_pack < t_plain:
-                    pick = Pk
+                key, best = ("taylor", 1, _lib.CPF), None
+                for form in (P, Pk, Pk.sliced()):
+                    if form is None:
+                        continue
+                    tune_taylor(form, 1, _lib.CPF)
+                    t = form.__dict__.get("_tuned_ms", {}).get(key)
+                    if t is not None and (best is None or t < best):
+                        pick, best = form, t
             self._pick = pick
         return pick, _lib.CPF
 

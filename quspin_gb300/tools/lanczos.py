@@ -23,7 +23,7 @@ from scipy.linalg import eigh_tridiagonal
 
 from .. import _device as D
 from .. import _lib
-from ..sparse import DeviceCSR, DeviceDIA, to_device_matrix
+from ..sparse import SLICED, DeviceCSR, DeviceDIA, to_device_matrix
 
 __all__ = ["lanczos_full", "lanczos_iter", "lin_comb_Q_T", "expm_lanczos", "FTLM_static_iteration",
            "LTLM_static_iteration"]
@@ -116,13 +116,17 @@ def _recurrence(op, q0, m, eps, Q=None, reorth=False):
         # below; so does lanczos_iter, whose second pass repeats that loop
         from ..tune import tune_spmv
         group = tune_spmv(M, 1, np.complex128 if cplx else np.float64, "double", operand=P)
+        indptr = M.indptr
+        if group & SLICED:
+            P = P.sliced()
+            indptr = P.indptr
         r = torch.empty_like(q0)
         xs, _ = M._pair_scratch(n2)
         scr = D.scratch_doubles(L.qs_lanczos_run_scratch_doubles(m, int(reorth)))
         ctl = torch.zeros(L.qs_lanczos_run_ctl_bytes() // 4, dtype=torch.int32, device=D.device())
         ctl[1] = m
         dv = lambda t: D.ptr(torch.view_as_real(t) if t.is_complex() else t)
-        _lib.check(L.qs_lanczos_run(n, m, cplx, float(eps), int(reorth), D.ptr(M.indptr), D.ptr(P.indices),
+        _lib.check(L.qs_lanczos_run(n, m, cplx, float(eps), int(reorth), D.ptr(indptr), D.ptr(P.indices),
                                     D.ptr(P.data), P.vcode, int(group), dv(Q), dv(r), D.ptr(xs), D.ptr(ab),
                                     D.ptr(scr), D.ptr(ctl), st), "qs_lanczos_run")
         m_eff = int(ctl[1].item())

@@ -5,7 +5,8 @@ U entries in flight per lane).  The best shape depends on the row-length
 distribution and on how the gathers of the vector spread over L2, so it is
 measured: a handful of candidate shapes around the nnz/row heuristic are timed
 with CUDA events on the actual matrix and the fastest is kept on the matrix
-object.  Matrices smaller than ``MIN_ROWS`` keep the heuristic shape.
+object.  For one vector on a packed operand its sliced form (csrc/sell.cu, one
+shape, launch code bit ``SLICED``) is timed with them.  Matrices smaller than ``MIN_ROWS`` keep the heuristic shape.
 """
 from __future__ import annotations
 
@@ -14,6 +15,7 @@ import torch
 
 from . import _device as D
 from . import _lib
+from .sparse import SLICED
 
 MIN_ROWS = 65536
 
@@ -105,6 +107,8 @@ def tune_spmv(M, nvec=1, xdtype=np.complex128, precision="double", operand=None)
     if (nvec == 1 and np.dtype(xdtype).kind == "c" and getattr(operand, "padded", False)
             and getattr(operand, "vcode", None) in (_lib.PF8P, _lib.CPF8P)):
         codes += [encode(G, 1) | (6 << 20) for G in (2, 4)]      # column words read four per load
+    if nvec == 1 and getattr(operand, "vcode", None) in (_lib.PF8P, _lib.CPF8P) and operand.sliced() is not None:
+        codes.append(encode(2, 1) | SLICED)
     for code in codes:
         t = _time(lambda: M.matvec_into(x, y, group=code, precision=precision, operand=operand))
         if best_t is None or t < best_t:
@@ -142,6 +146,8 @@ def tune_taylor(M, nvec, btype):
         cands += [(2, 2, 1 << 4)]     # the vectors-across-lanes kernel (csrc/expm_vl.cu)
     if getattr(M, "vcode", None) in (_lib.PF8P, _lib.CPF8P):
         cands = []                 # the packed form runs only in the single-vector kernels
+    if getattr(M, "vcode", None) in (_lib.PF8S, _lib.CPF8S):
+        cands = [(2, 2, SLICED >> 16)]
     cands += [({1: 4, 2: 2, 3: 8, 4: 2, 5: 4, 6: 2, 7: 4}[shape], 2, (shape << 4) | (occ << 2))
               for shape, occ in r32_candidates(M, nvec, btype)]
     for G, U, ch in cands:

@@ -1,0 +1,146 @@
+"""The sliced operand and its single-vector kernels (csrc/sell.cu): the words
+of every row survive the re-ordering, at slice edges, with empty, even, uneven
+and over-long rows; the product, the Taylor term and the Lanczos product against
+the row hand-out kernels on the same packed operand; padding never reads into
+a result.
+
+Tolerance: the same float-pair products summed in another order, 48-bit
+roundings over at most 128 nonzeros: 1e-13 of the row's absolute sum."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(n, cplx, kind, rng):
+    m = min(n, 9)
+    if kind == "uneven":                                  # empty rows among rows of up to 12
+        lens = rng.integers(0, min(n, 12) + 1, n)
+    elif kind == "long":
+        lens = np.full(n, min(n, 128))
+    else:
+        lens = np.full(n, m)
+    cols = [np.sort(rng.choice(n, l, replace=False)) for l in lens]
+    ip = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    vals = rng.choice(np.array([0.5, -1.25, 2.0, 1.0 / 3.0]), ip[-1])
+    if cplx:
+        vals = vals * rng.choice(np.array([1.0, 1j, 0.6 + 0.8j]), ip[-1])
+    return sp.csr_matrix((vals, np.concatenate(cols) if ip[-1] else np.zeros(0, np.int32), ip), shape=(n, n))
+
+
+def _packed(A):
+    from quspin_gb300.sparse import DeviceCSR
+    M = DeviceCSR.from_scipy(A)
+    return M, M.paired().packed()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 1024, 5000])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("kind", ["even", "uneven", "long"])
+def test_sliced_words_and_product(cuda, n, cplx, kind):
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300.sparse import SLICED, SlicedCSR
+    from quspin_gb300.tune import encode
+    rng = np.random.default_rng(n + 7 * cplx + len(kind))
+    A = _matrix(n, cplx, kind, rng)
+    if A.nnz == 0:
+        pytest.skip("no nonzeros")
+    M, P = _packed(A)
+    limit, SlicedCSR.MAX_PADDING = SlicedCSR.MAX_PADDING, 40.0
+    try:
+        S = P.sliced()
+    finally:
+        SlicedCSR.MAX_PADDING = limit
+    # every row's words, as a set, and nothing else
+    sptr, words = D.to_host(S.indptr), D.to_host(S.indices).view(np.uint32)
+    src = D.to_host(P.indices).view(np.uint32)
+    for s in range((n + 31) // 32):
+        block = words[sptr[s] * 128:sptr[s + 1] * 128].reshape(-1, 32, 4)
+        for lane in range(32):
+            got = block[:, lane, :].reshape(-1)
+            got = np.sort(got[got != 0xffffffff])
+            r = s * 32 + lane
+            want = src[A.indptr[r]:A.indptr[r + 1]] if r < n else src[:0]
+            np.testing.assert_array_equal(got, np.sort(want))
+    group = encode(2, 1)
+    for xc in ([True] if cplx else [False, True]):
+        x = rng.normal(size=n) + (1j * rng.normal(size=n) if xc else 0.0)
+        xd = D.to_device(x)
+        scale = abs(A) @ np.abs(x) + 1e-300
+        for a, over in ((1.0, True), ((0.3 - 0.7j) if xc else -0.7, False)):
+            y0 = rng.normal(size=n) + (1j * rng.normal(size=n) if xc else 0.0)
+            y1, y2 = D.to_device(y0.astype(x.dtype)), D.to_device(y0.astype(x.dtype))
+            M.matvec_into(xd, y1, a=a, overwrite=over, group=group, precision="double", operand=P)
+            M.matvec_into(xd, y2, a=a, overwrite=over, group=group | SLICED, precision="double", operand=P)
+            y1, y2 = D.to_host(y1), D.to_host(y2)
+            assert (np.abs(y1 - y2) <= 1e-13 * (scale + np.abs(y0))).all()
+    # a PAD reads column 0 and adds nothing: infinity there stays in the rows that hold it
+    x = np.ones(n, complex)
+    x[0] = np.inf
+    y = D.to_device(np.zeros(n, complex))
+    M.matvec_into(D.to_device(x), y, group=group | SLICED, precision="double", operand=P)
+    holds = np.asarray((A[:, 0] != 0).todense()).ravel()
+    assert np.isfinite(D.to_host(y)[~holds]).all()
+
+
+def test_sliced_refused(cuda):
+    rng = np.random.default_rng(0)
+    n = 4000
+    A = sp.random(n, n, density=0.0005, random_state=rng, format="lil")
+    A[5, :129] = 1.0                                        # one row too long for a slice
+    A = A.tocsr()
+    A.data = rng.choice(np.array([1.0, 2.0]), A.nnz)
+    assert _packed(A)[1].sliced() is None
+    rows = np.arange(0, n, 32)                              # one long row in every slice
+    C = sp.csr_matrix((np.ones(rows.size * 100), (np.repeat(rows, 100), np.tile(np.arange(100), rows.size))), shape=(n, n))
+    assert _packed(sp.csr_matrix(C + sp.eye(n)))[1].sliced() is None
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n", [1000, 70001])
+def test_sliced_evolution_and_lanczos(cuda, cplx, n):
+    """A whole evolution and a Lanczos run on the sliced form against the row
+    hand-out forms: the same partition and stopping, states within 1e-13, the
+    recurrence's coefficients within 1e-12 of its norm."""
+    import torch
+    from quspin_gb300 import _lib
+    from quspin_gb300 import _device as D
+    from quspin_gb300.sparse import SLICED, DeviceCSR
+    from quspin_gb300.tools import ExpmMultiplyParallel, lanczos_full
+    from quspin_gb300.tune import encode
+    rng = np.random.default_rng(n + cplx)
+    A = _matrix(n, cplx, "even", rng)
+    A = sp.csr_matrix(A + A.conj().T)
+    A.sum_duplicates()
+    v = rng.normal(size=n) + 1j * rng.normal(size=n)
+    v /= np.linalg.norm(v)
+    old, ExpmMultiplyParallel.SMALL_MAX_ROWS = ExpmMultiplyParallel.SMALL_MAX_ROWS, 0
+    try:
+        out, terms = [], []
+        for sliced in (False, True):
+            op = ExpmMultiplyParallel(DeviceCSR.from_scipy(A), a=-0.4j)
+            P = op.A_device.paired().packed()
+            code = encode(2, 2) | (4 << 20)
+            if sliced:
+                P, code = P.sliced(), encode(2, 2) | SLICED
+            op._pick = P
+            P.__dict__.setdefault("_tuned", {})[("taylor", 1, _lib.CPF)] = code
+            F = D.to_device(v * 1e150)
+            op.run_device(F)
+            out.append(D.to_host(F) / 1e150)
+            terms.append(op.terms_executed)
+    finally:
+        ExpmMultiplyParallel.SMALL_MAX_ROWS = old
+    assert np.linalg.norm(out[1] - out[0]) <= 1e-13 * np.linalg.norm(out[0])
+    assert terms[0] == terms[1]
+    E = []
+    m = 12
+    for sliced in (False, True):
+        M = DeviceCSR.from_scipy(A)
+        P = M.paired().packed()
+        key = ("spmv", 1, np.dtype(np.complex128).str, "double", P.vcode)
+        M._tuned = {key: encode(2, 1) | (SLICED if sliced else 0)}
+        E.append(lanczos_full(M, D.to_device(v), m)[0])
+    assert np.abs(E[1] - E[0]).max() <= 1e-12 * np.abs(E[0]).max()
