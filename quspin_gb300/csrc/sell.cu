@@ -18,8 +18,9 @@
 // the product of a complex vector, its split into pairs included, 506 -> 383,
 // 140 -> 112 and 50 -> 43 us, Ising L = 22 31 -> 29, XXZ L = 26 (rows of 5 to 27)
 // 26 -> 25.  Re-ordering takes 4.9 ms at 159 M nonzeros, once per operator.
-// Bound at L = 30 by issue slots (68%) and L1 (59%) about alike, at L = 32 by the
-// re-reading of the vector, which with the streams exceeds L2.
+// Bound by issue slots (68%) and L1 (59%) about alike.  DRAM traffic of a term at
+// L = 32, where the term vectors, F and the words exceed L2 together: 1.98 -> 1.04
+// GB, 1.02 times what the padded words and the vectors once come to.
 //
 // Words: col << 8 | code as in the packed form, PAD where a row has no nonzero
 // in the slot; slots in groups of four, a group as 32 x 16 bytes, so that a

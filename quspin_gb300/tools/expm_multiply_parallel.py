@@ -215,9 +215,10 @@ class ExpmMultiplyParallel:
 
     def _operand(self, nvec=1):
         """(matrix in the value form of the precision, B storage code).  For
-        one vector in the float-pair form, the coded operand, its packed form
-        (code bytes inside the column words) and that in slices are tuned once
-        and the fastest is kept."""
+        one vector in the float-pair form, the packed form of the coded operand
+        (code bytes inside the column words) and that in slices, or where rows
+        do not fit slices the coded operand itself, are tuned once and the
+        faster is kept."""
         if self._precision == "mixed":
             return self._mixed_matrix(), _lib.C64
         if self._precision == "ieee":
@@ -231,10 +232,9 @@ class ExpmMultiplyParallel:
             Pk = P.packed() if P.shape[0] >= 65536 else None
             if Pk is not None:
                 from ..tune import tune_taylor
+                S = Pk.sliced()
                 key, best = ("taylor", 1, _lib.CPF), None
-                for form in (P, Pk, Pk.sliced()):
-                    if form is None:
-                        continue
+                for form in (P, Pk) if S is None else (Pk, S):
                     tune_taylor(form, 1, _lib.CPF)
                     t = form.__dict__.get("_tuned_ms", {}).get(key)
                     if t is not None and (best is None or t < best):

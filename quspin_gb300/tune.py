@@ -72,6 +72,11 @@ def lanes_operand(M, nvec, code):
     return M if P is None else P
 
 
+def _sliced(M):
+    """The sliced form of a packed operand, or None."""
+    return M.sliced() if getattr(M, "vcode", None) in (_lib.PF8P, _lib.CPF8P) else None
+
+
 def _time(fn, reps=5):
     st = torch.cuda.current_stream()
     for _ in range(2):
@@ -107,7 +112,9 @@ def tune_spmv(M, nvec=1, xdtype=np.complex128, precision="double", operand=None)
     if (nvec == 1 and np.dtype(xdtype).kind == "c" and getattr(operand, "padded", False)
             and getattr(operand, "vcode", None) in (_lib.PF8P, _lib.CPF8P)):
         codes += [encode(G, 1) | (6 << 20) for G in (2, 4)]      # column words read four per load
-    if nvec == 1 and getattr(operand, "vcode", None) in (_lib.PF8P, _lib.CPF8P) and operand.sliced() is not None:
+    if nvec == 1 and _sliced(operand) is not None:
+        # against the row hand-out shapes that win where rows share few lines
+        codes = [c for c in codes if c >> 20] or [encode(G, U) for G in (2, 4) for U in (1, 2)]
         codes.append(encode(2, 1) | SLICED)
     for code in codes:
         t = _time(lambda: M.matvec_into(x, y, group=code, precision=precision, operand=operand))
@@ -148,8 +155,13 @@ def tune_taylor(M, nvec, btype):
         cands = []                 # the packed form runs only in the single-vector kernels
     if getattr(M, "vcode", None) in (_lib.PF8S, _lib.CPF8S):
         cands = [(2, 2, SLICED >> 16)]
+    rows = r32_candidates(M, nvec, btype)
+    if nvec == 1 and _sliced(M) is not None:
+        # the form to beat is the sliced one: time the shapes that win where
+        # rows share few lines (all of them cost 0.28 s at 159 M nonzeros)
+        rows = [c for c in rows if c in ((4, 1), (6, 1), (6, 2))]
     cands += [({1: 4, 2: 2, 3: 8, 4: 2, 5: 4, 6: 2, 7: 4}[shape], 2, (shape << 4) | (occ << 2))
-              for shape, occ in r32_candidates(M, nvec, btype)]
+              for shape, occ in rows]
     for G, U, ch in cands:
         code = encode(G, U) | (ch << 16)
         A = lanes_operand(M, nvec, code)

@@ -144,3 +144,36 @@ def test_sliced_evolution_and_lanczos(cuda, cplx, n):
         M._tuned = {key: encode(2, 1) | (SLICED if sliced else 0)}
         E.append(lanczos_full(M, D.to_device(v), m)[0])
     assert np.abs(E[1] - E[0]).max() <= 1e-12 * np.abs(E[0]).max()
+
+
+@pytest.mark.parametrize("kind", ["even", "uneven"])
+def test_tuned_pick(cuda, kind):
+    """At tuned sizes the evolution takes the sliced or the packed form where
+    slices apply, else a row hand-out form, with the same result."""
+    from quspin_gb300 import _lib
+    from quspin_gb300 import _device as D
+    from quspin_gb300.sparse import DeviceCSR
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    from quspin_gb300.tune import encode
+    rng = np.random.default_rng(3)
+    n = 66001
+    A = _matrix(n, False, kind, rng)
+    if kind == "uneven":                                    # a row of 100 in every slice
+        rows = np.arange(0, n, 32)
+        A = A + sp.csr_matrix((np.ones(100 * rows.size), (np.repeat(rows, 100), np.tile(np.arange(100) * 7, rows.size))),
+                              shape=(n, n))
+    A = sp.csr_matrix(A + A.T)
+    v = rng.normal(size=n) + 1j * rng.normal(size=n)
+    v /= np.linalg.norm(v)
+    op = ExpmMultiplyParallel(DeviceCSR.from_scipy(A), a=-0.1j)
+    op.set_partition(8, 2)
+    P, _ = op._operand(1)
+    assert (op.A_device.paired().packed().sliced() is None) == (kind == "uneven")
+    sliced = (_lib.PF8P, _lib.PF8S)
+    assert P.vcode in (sliced if kind == "even" else (_lib.PF8, _lib.PF8P))
+    out = D.to_host(op.dot(D.to_device(v)))
+    ref = ExpmMultiplyParallel(DeviceCSR.from_scipy(A), a=-0.1j)
+    ref.set_partition(8, 2)
+    ref._pick = ref.A_device.paired()
+    ref._pick.__dict__.setdefault("_tuned", {})[("taylor", 1, _lib.CPF)] = encode(4, 1)
+    assert np.linalg.norm(out - D.to_host(ref.dot(D.to_device(v)))) <= 1e-13 * np.linalg.norm(out)
