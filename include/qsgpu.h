@@ -185,6 +185,13 @@ int qs_expm_multiply(int64_t n, int64_t nnz, const void *d_indptr, int idx64, co
                      const void *d_data, int dtype, void *d_F, int64_t nvec, int s, int m_star, double tol,
                      double mu_re, double mu_im, const void *d_coeff, const void *d_eta, const void *d_one,
                      void *d_work, int btype, void *d_ctl, int group, void *stream);
+/* Values with at most 256 distinct ones as a sorted table d_vals (256 doubles,
+ * or 256 complex) and one code byte each.  d_state: qs_value_codes_state_bytes()
+ * of device memory; its first two int32 receive whether the values cannot be
+ * coded (too many distinct ones, or a NaN) and the number of distinct values. */
+int qs_value_codes_state_bytes(void);
+int qs_value_codes(int64_t count, const double *d_src, int cplx, double *d_vals, unsigned char *d_codes, void *d_state,
+                   void *stream);
 /* The sliced form of a packed coded matrix (types 10 / 11: one vector, 32 rows
  * per slice, slots in groups of four) for qs_csr_matvec_pairs, qs_taylor_term,
  * qs_expm_multiply and qs_lanczos_run; its slice pointers (int64, groups before

@@ -304,13 +304,26 @@ class DeviceDIA:
         return self.tocsr().diagonal().sum()
 
 
+def _device_codes(src):
+    count, cplx = src.numel(), int(src.is_complex())
+    vals = torch.empty((256, 2) if cplx else 256, dtype=torch.float64, device=src.device)
+    codes = torch.empty(count, dtype=torch.uint8, device=src.device)
+    state = torch.empty(_lib.load().qs_value_codes_state_bytes(), dtype=torch.uint8, device=src.device)
+    _lib.call("qs_value_codes", count, D.ptr(src), cplx, D.ptr(vals), D.ptr(codes), D.ptr(state), D.stream())
+    over, distinct = state[:8].view(torch.int32).tolist()
+    return None if over else (vals, codes, distinct)
+
+
 def value_codes(src, table=256):
     """The coded form of a value array: (vals, codes, distinct) with vals the
     table padded with zeros to ``table`` entries (float64 [table], or
     [table, 2] real / imaginary parts for complex src), codes uint8 with
     vals[codes] == src exactly, or None when src has more than ``table``
-    distinct values (or a NaN).  Only one-dimensional sorts: complex values
-    are coded by the pair of their real- and imaginary-part codes."""
+    distinct values (or a NaN).  Device arrays of doubles go through
+    csrc/codes.cu; others through one-dimensional sorts, complex values by the
+    pair of their real- and imaginary-part codes."""
+    if src.is_cuda and table == 256 and src.dtype in (torch.float64, torch.complex128) and src.numel() > 0:
+        return _device_codes(src.contiguous())
     if src.numel() == 0 or bool(torch.isnan(torch.view_as_real(src) if src.is_complex() else src).any()):
         return None
     if src.is_complex():
