@@ -119,7 +119,8 @@ def profile_traffic(kernel):
                 recs[-1][key] = line.split(":", 1)[1].strip()
     rec = next((r for r in recs if r.get("traffic_kernel") == kernel), recs[0] if recs else {})
     if rec.get("traffic_kernel") != kernel:
-        return None, "the ncu summary covers {}, not {}".format(rec.get("traffic_kernel"), kernel)
+        return None, "the ncu summary covers {}, not {}".format(
+            " and ".join(sorted(r["traffic_kernel"] for r in recs if "traffic_kernel" in r)) or None, kernel)
     if rec.get("traffic_source_sha256") != kernel_source_sha(kernel):
         return None, "the kernel's sources changed since the ncu capture"
     try:
@@ -627,7 +628,9 @@ def run_ours(args, rank, ws):
         # timings are distorted under a profiler)
         from quspin_gb300 import _lib
         P0 = A.paired()
-        Mp = P0.packed() if (args.taylor_code >> 20) & 7 and P0.packed() is not None else P0
+        Mp = P0.packed() if (args.taylor_code >> 20) & 15 and P0.packed() is not None else P0
+        if (args.taylor_code >> 23) & 1:
+            Mp = Mp.sliced()
         Mp.__dict__.setdefault("_tuned", {})[("taylor", 1, _lib.CPF)] = int(args.taylor_code)
         op._pick = Mp
     rng = np.random.default_rng(0)

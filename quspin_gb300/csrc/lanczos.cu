@@ -470,9 +470,10 @@ extern "C" int64_t qs_lanczos_run_scratch_doubles(int m, int reorth)
 // reorth: classical Gram-Schmidt against all earlier rows, a second pass when
 // the first lost more than 1 - 1/sqrt(2) of the norm, decided on the device.
 // pdtype: plain pairs (QS_PF / QS_CPF) or packed codes (QS_PF8P / QS_CPF8P),
-// int32 indptr; group: launch shape of the product.  r: n elements; xs: n split
-// elements (8 or 16 bytes each); ab: a[m], b[m]; ctl: qs_lanczos_run_ctl_bytes
-// of zeros with m_eff (the second word) set to m.
+// int32 indptr, or the sliced form (csrc/sell.cuh; indptr: its slice pointers);
+// group: launch shape of the product.  r: n elements; xs: n split elements (8 or
+// 16 bytes each); ab: a[m], b[m]; ctl: qs_lanczos_run_ctl_bytes of zeros with
+// m_eff (the second word) set to m.
 extern "C" int qs_lanczos_run(int64_t n, int m, int cplx, double eps, int reorth, const int32_t *indptr,
                               const int32_t *indices, const void *pdata, int pdtype, int group, double *Q, double *r,
                               void *xs, double *ab, double *scratch, void *ctl, void *stream)

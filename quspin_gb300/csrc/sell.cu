@@ -18,7 +18,7 @@
 // the product of a complex vector, its split into pairs included, 506 -> 383,
 // 140 -> 112 and 50 -> 43 us, Ising L = 22 31 -> 29, XXZ L = 26 (rows of 5 to 27)
 // 26 -> 25.  Re-ordering takes 4.9 ms at 159 M nonzeros, once per operator.
-// Bound by issue slots (68%) and L1 (59%) about alike.  DRAM traffic of a term at
+// Bound by issue slots (66%) and L1 (65%) about alike.  DRAM traffic of a term at
 // L = 32, where the term vectors, F and the words exceed L2 together: 1.98 -> 1.04
 // GB, 1.02 times what the padded words and the vectors once come to.
 //
