@@ -241,13 +241,31 @@ extern "C" int qs_sym_destroy(void *h)
 
 static size_t sym_smem(const QsSym *q) { return q->staged_bytes(); }
 
+// Shared memory a block may use, static and dynamic together.
+static size_t block_smem_max()
+{
+    static int most = 0;
+    if (!most) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || most <= 0)
+            most = 48 * 1024;
+    }
+    return (size_t)most;
+}
+
+// Both bounds, 48 KB without asking and block_smem_max() with it, count the
+// kernel's static shared memory too (none has more than 16 KB).
 template <typename K>
 static int set_smem(K kernel, size_t bytes)
 {
-    if (bytes > 48 * 1024) {
-        if (bytes > 220 * 1024) return QS_ERR_UNSUPPORTED;
+    if (bytes <= 32 * 1024) return QS_OK;
+    cudaFuncAttributes at;
+    QS_CHECK(cudaFuncGetAttributes(&at, kernel));
+    const size_t all = bytes + at.sharedSizeBytes;
+    if (all > block_smem_max()) return QS_ERR_UNSUPPORTED;
+    if (all > 48 * 1024)
         QS_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    }
     return QS_OK;
 }
 
@@ -399,13 +417,13 @@ __device__ __forceinline__ void binom_table(int n, int k, uint64_t *c)
 }
 
 // word number `rank` (ascending) of the n-bit words with k set bits; c: the
-// binom_table with rows of `width` words, at least n rows
+// binom_table with rows of `width` words, at least n rows (null: computed)
 template <typename S>
 __device__ __forceinline__ S unrank_comb(int n, int k, uint64_t rank, const uint64_t *c, int width)
 {
     S s = 0;
     for (int b = n - 1; b >= 0 && k > 0; b--) {
-        const uint64_t m = c[b * width + k];
+        const uint64_t m = c ? c[b * width + k] : binom_u64(b, k);
         if (rank >= m) { s |= (S)1 << b; rank -= m; k--; }
     }
     return s;
@@ -424,7 +442,7 @@ __device__ __forceinline__ S gosper_next(S s)
 
 struct EnumArgs {
     int kind, p0, p1, half;
-    int bin_n, bin_k;     // rows and largest column of the binomial table
+    int bin_n, bin_k;     // rows (0: no table) and largest column of the binomial table
     uint64_t total, n_lo;
     int64_t nchunks;
 };
@@ -443,27 +461,37 @@ struct EnumArgs {
 // Measured at L = 28, Sz = 0, k = 0, p = z = +1 (40.1 M candidates, 112
 // elements): 4.76 ms a pass with full checks in step and byte tables, 0.82 ms so
 // (issue slots 67% busy).
+//
+// Queues, map tables and binomials share the block's dynamic memory; what
+// does not fit there (a dozen maps from byte tables at 64 sites) gives way
+// first in the binomials, then in the warps (enum_fit).
 #define ENUM_WARPS 4
+
+template <typename S>
+struct EnumQueue {
+    S state[64];
+    int found[32];              // representatives of each lane's chunk so far
+    unsigned char lane[64];
+};
 
 template <typename S, int PASS>
 __global__ void __launch_bounds__(32 * ENUM_WARPS) enum_kernel(const __grid_constant__ SymParams<S> P, EnumArgs A, int64_t *__restrict__ off,
                                                                S *__restrict__ states, uint32_t *__restrict__ norms,
                                                                size_t tab_elems)
 {
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ S q_state[ENUM_WARPS][64];
-    __shared__ unsigned char q_lane[ENUM_WARPS][64];
-    __shared__ int found[ENUM_WARPS][32];
-    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    EnumQueue<S> &Q = reinterpret_cast<EnumQueue<S> *>(smem_raw)[wib];
+    unsigned char *tables = smem_raw + nwarps * sizeof(EnumQueue<S>);
+    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(tables), tab_elems);
     const unsigned lt = (1u << lane) - 1u;
-    uint64_t *bin = reinterpret_cast<uint64_t *>(smem_raw + ((tab_elems * sizeof(S) + 7) & ~(size_t)7));
+    uint64_t *bin = A.bin_n ? reinterpret_cast<uint64_t *>(tables + ((tab_elems * sizeof(S) + 7) & ~(size_t)7)) : nullptr;
     const int width = A.bin_k + 1;
     binom_table(A.bin_n, A.bin_k, bin);
     const S lo_full = A.kind == 2 ? (S)((uint64_t)1 << A.half) : (S)0;
     const S min_lo = (A.kind == 2 && A.p1 > 0) ? (S)(((uint64_t)1 << A.p1) - 1) : (S)0;
-    const int64_t nw = (int64_t)gridDim.x * ENUM_WARPS;
-    for (int64_t cb = ((int64_t)blockIdx.x * ENUM_WARPS + wib) * 32; cb < A.nchunks; cb += nw * 32) {
+    const int64_t nw = (int64_t)gridDim.x * nwarps;
+    for (int64_t cb = ((int64_t)blockIdx.x * nwarps + wib) * 32; cb < A.nchunks; cb += nw * 32) {
         const int64_t ch = cb + lane;
         uint64_t len = 0;
         S s = 0, hi = 0, lo = 0;
@@ -481,7 +509,7 @@ __global__ void __launch_bounds__(32 * ENUM_WARPS) enum_kernel(const __grid_cons
             }
         }
         const int64_t wend = (PASS && ch < A.nchunks) ? off[ch + 1] : 0;
-        found[wib][lane] = 0;
+        Q.found[lane] = 0;
         int qn = 0;
         for (int t = 0; t <= ENUM_CH; t++) {
             // the last round only empties the queue
@@ -490,21 +518,21 @@ __global__ void __launch_bounds__(32 * ENUM_WARPS) enum_kernel(const __grid_cons
             const unsigned bal = __ballot_sync(0xffffffffu, pass);
             if (pass) {
                 const int at = qn + __popc(bal & lt);
-                q_state[wib][at] = s;
-                q_lane[wib][at] = (unsigned char)lane;
+                Q.state[at] = s;
+                Q.lane[at] = (unsigned char)lane;
             }
             qn += __popc(bal);
             __syncwarp();
             while (qn >= 32 || (t == ENUM_CH && qn > 0)) {
                 const int take = qn < 32 ? qn : 32;
-                const S c = q_state[wib][lane];
-                const int who = lane < take ? (int)q_lane[wib][lane] : 32 + lane;
+                const S c = Q.state[lane];
+                const int who = lane < take ? (int)Q.lane[lane] : 32 + lane;
                 const double nv = lane < take ? check_state(V, c) : 0.0;
                 const bool hit = nv > 0.0;
                 // earlier entries of the same chunk in this batch come first
                 const unsigned same = __match_any_sync(0xffffffffu, who);
                 const unsigned hits = __ballot_sync(0xffffffffu, hit) & same;
-                const int before = lane < take ? found[wib][who] : 0;
+                const int before = lane < take ? Q.found[who] : 0;
                 const int64_t end = PASS ? __shfl_sync(0xffffffffu, wend, who & 31) : 0;
                 __syncwarp();
                 if (hit) {
@@ -513,13 +541,13 @@ __global__ void __launch_bounds__(32 * ENUM_WARPS) enum_kernel(const __grid_cons
                         states[end - 1 - rank] = c;
                         norms[end - 1 - rank] = (uint32_t)nv;
                     }
-                    if (!(hits & ~lt & ~(1u << lane))) found[wib][who] = rank + 1;   // the batch's last of its chunk
+                    if (!(hits & ~lt & ~(1u << lane))) Q.found[who] = rank + 1;   // the batch's last of its chunk
                 }
                 const int left = qn - take;      // < 32
-                const S ms = q_state[wib][32 + lane];
-                const unsigned char ml = q_lane[wib][32 + lane];
+                const S ms = Q.state[32 + lane];
+                const unsigned char ml = Q.lane[32 + lane];
                 __syncwarp();
-                if (lane < left) { q_state[wib][lane] = ms; q_lane[wib][lane] = ml; }
+                if (lane < left) { Q.state[lane] = ms; Q.lane[lane] = ml; }
                 qn = left;
                 __syncwarp();
             }
@@ -534,7 +562,7 @@ __global__ void __launch_bounds__(32 * ENUM_WARPS) enum_kernel(const __grid_cons
                 }
             }
         }
-        if (!PASS && ch < A.nchunks) off[ch + 1] = found[wib][lane];
+        if (!PASS && ch < A.nchunks) off[ch + 1] = Q.found[lane];
         __syncwarp();
     }
 }
@@ -552,6 +580,20 @@ static int enum_setup(const QsSym *q, int kind, int p0, int p1, EnumArgs &A)
     if (kind == 1 && (p0 < 0 || p0 > q->N)) return QS_ERR_ARG;
     if (kind == 2 && (q->N % 2 || p0 < 0 || p1 < 0 || p0 > q->N / 2 || p1 > q->N / 2)) return QS_ERR_ARG;
     return QS_OK;
+}
+
+// Warps per block (0: none fit) and dynamic shared memory of the enumeration;
+// drops the binomial table where it does not fit.
+static int enum_fit(const QsSym *q, EnumArgs &A, size_t &smem)
+{
+    const size_t queue = q->sbytes == 4 ? sizeof(EnumQueue<uint32_t>) : sizeof(EnumQueue<uint64_t>);
+    const size_t tables = (sym_smem(q) + 7) & ~(size_t)7, bin = sizeof(uint64_t) * A.bin_n * (A.bin_k + 1);
+    smem = ENUM_WARPS * queue + tables + bin;
+    if (smem <= block_smem_max()) return ENUM_WARPS;
+    A.bin_n = 0;
+    for (int w = ENUM_WARPS; w > 0; w >>= 1)
+        if ((smem = w * queue + tables) <= block_smem_max()) return w;
+    return 0;
 }
 
 extern "C" int64_t qs_enum_num_chunks(int N, int kind, int p0, int p1)
@@ -576,8 +618,9 @@ extern "C" int qs_enum_count(void *sym, int kind, int p0, int p1, int64_t *off, 
     if (nchunks != A.nchunks) return QS_ERR_ARG;
     cudaStream_t st = qs_stream(stream);
     QS_CHECK(cudaMemsetAsync(off, 0, sizeof(int64_t), st));
-    const size_t sm = ((sym_smem(q) + 7) & ~(size_t)7) + sizeof(uint64_t) * A.bin_n * (A.bin_k + 1);
-    int blocks = qs_num_sms() * 8, threads = 32 * ENUM_WARPS;
+    size_t sm;
+    const int blocks = qs_num_sms() * 8, threads = 32 * enum_fit(q, A, sm);
+    if (!threads) return QS_ERR_UNSUPPORTED;
     if (q->sbytes == 4) {
         auto k = enum_kernel<uint32_t, 0>;
         if ((rc = set_smem(k, sm))) return rc;
@@ -607,8 +650,9 @@ extern "C" int qs_enum_write(void *sym, int kind, int p0, int p1, const int64_t 
     if (rc) return rc;
     if (nchunks != A.nchunks) return QS_ERR_ARG;
     cudaStream_t st = qs_stream(stream);
-    const size_t sm = ((sym_smem(q) + 7) & ~(size_t)7) + sizeof(uint64_t) * A.bin_n * (A.bin_k + 1);
-    int blocks = qs_num_sms() * 8, threads = 32 * ENUM_WARPS;
+    size_t sm;
+    const int blocks = qs_num_sms() * 8, threads = 32 * enum_fit(q, A, sm);
+    if (!threads) return QS_ERR_UNSUPPORTED;
     if (q->sbytes == 4) {
         auto k = enum_kernel<uint32_t, 1>;
         if ((rc = set_smem(k, sm))) return rc;
@@ -716,7 +760,7 @@ template <typename S>
 __global__ void rep_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, const S *__restrict__ in, int64_t n, S *__restrict__ out,
                            int32_t *__restrict__ g_out, int8_t *__restrict__ sign_out)
 {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int g[QS_MAXMAPS];
@@ -755,7 +799,7 @@ extern "C" int qs_representative(void *sym, const void *states, int64_t n, void 
 template <typename S>
 __global__ void norm_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, const S *__restrict__ in, int64_t n, uint32_t *__restrict__ out)
 {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = (uint32_t)check_state(V, in[i]);
@@ -986,6 +1030,8 @@ __device__ __forceinline__ int64_t term_element(const SymView<S> &V, const Basis
 // Measured at L = 28 (358 k kets, 112 hopping terms, 112 elements): a count or
 // fill pass 6.9 ms with one search per thread and term, 0.95 ms so (integer
 // pipe 74% busy); the matrix-free apply at L = 26 2.22 ms before, 0.29 ms now.
+// The queues lie before the map tables in the block's dynamic memory; where
+// both do not fit, the block has fewer warps (elem_launch).
 #define ELEM_WARPS 4
 
 template <typename S>
@@ -1004,9 +1050,8 @@ __device__ __forceinline__ void for_elements(const SymView<S> &V, const BasisVie
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int64_t groups = (B.Ns + 31) / 32, tasks = groups * nslice;
-    const int per = (TV.T + nslice - 1) / nslice;
-    for (int64_t w = (int64_t)blockIdx.x * ELEM_WARPS + (threadIdx.x >> 5); w < tasks;
-         w += (int64_t)gridDim.x * ELEM_WARPS) {
+    const int per = (TV.T + nslice - 1) / nslice, nwarps = blockDim.x >> 5;
+    for (int64_t w = (int64_t)blockIdx.x * nwarps + (threadIdx.x >> 5); w < tasks; w += (int64_t)gridDim.x * nwarps) {
         const int64_t kb = w / nslice * 32, i = kb + lane;
         const int t0 = (int)(w % nslice) * per, t1 = t0 + per < TV.T ? t0 + per : TV.T;
         const bool valid = i < B.Ns;
@@ -1092,7 +1137,7 @@ template <typename S>
 __global__ void op_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, BasisView B, TermView TV, int64_t *__restrict__ row,
                           int64_t *__restrict__ col, double *__restrict__ ME, int *__restrict__ d_err)
 {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
     int err = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < B.Ns; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1162,9 +1207,9 @@ __global__ void __launch_bounds__(32 * ELEM_WARPS)
 csr_count_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, BasisView B, TermView TV, int nslice, int64_t *__restrict__ rowcnt,
                  int *__restrict__ term_flags, int *__restrict__ d_err)
 {
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ ElemQueue<S> queue[ELEM_WARPS];
-    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ElemQueue<S> *queue = reinterpret_cast<ElemQueue<S> *>(smem_raw);
+    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(queue + (blockDim.x >> 5)), tab_elems);
     int err = 0;
     for_elements(V, B, TV, nslice, queue[threadIdx.x >> 5], err,
                  [&](int t, int64_t i, int64_t j, double re, double im) {
@@ -1183,9 +1228,9 @@ csr_fill_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, BasisV
                 const int64_t *__restrict__ rowptr, int64_t *__restrict__ cursor, uint64_t *__restrict__ keys,
                 T *__restrict__ vals, int *__restrict__ d_err)
 {
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ ElemQueue<S> queue[ELEM_WARPS];
-    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ElemQueue<S> *queue = reinterpret_cast<ElemQueue<S> *>(smem_raw);
+    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(queue + (blockDim.x >> 5)), tab_elems);
     int err = 0;
     for_elements(V, B, TV, nslice, queue[threadIdx.x >> 5], err,
                  [&](int t, int64_t i, int64_t j, double re, double im) {
@@ -1203,7 +1248,7 @@ template <typename S, typename T>
 __global__ void csr_diag_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, BasisView B, TermView TV, T *__restrict__ diag,
                                 int *__restrict__ term_flags, int *__restrict__ d_err)
 {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
     int err = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < B.Ns; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1345,10 +1390,18 @@ static int elem_slices(int64_t Ns, int T)
     int64_t s = (want + groups - 1) / groups, most = (T + 7) / 8;
     return (int)(s < 1 ? 1 : (s > most ? (most < 1 ? 1 : most) : s));
 }
-static int elem_blocks(int64_t Ns, int nslice)
+struct ElemLaunch {
+    int slices, blocks, threads;     // threads 0: the tables leave no room for a warp's queue
+    size_t smem;
+};
+static ElemLaunch elem_launch(const QsSym *q, int64_t Ns, int T)
 {
-    const int64_t b = ((Ns + 31) / 32 * nslice + ELEM_WARPS - 1) / ELEM_WARPS, cap = (int64_t)qs_num_sms() * 64;
-    return (int)(b < 1 ? 1 : (b > cap ? cap : b));
+    const size_t queue = q->sbytes == 4 ? sizeof(ElemQueue<uint32_t>) : sizeof(ElemQueue<uint64_t>);
+    int warps = ELEM_WARPS;
+    while (warps && warps * queue + sym_smem(q) > block_smem_max()) warps >>= 1;
+    const int slices = elem_slices(Ns, T);
+    const int64_t b = warps ? ((Ns + 31) / 32 * slices + warps - 1) / warps : 1, cap = (int64_t)qs_num_sms() * 64;
+    return {slices, (int)(b < 1 ? 1 : (b > cap ? cap : b)), 32 * warps, warps * queue + sym_smem(q)};
 }
 
 template <typename S>
@@ -1363,18 +1416,18 @@ template <typename T>
 static int csr_count_t(const QsSym *q, const BasisView &B, const TermView &TV, int64_t *rowcnt, int *flags,
                        int *d_err, cudaStream_t st)
 {
-    size_t sm = sym_smem(q);
+    const ElemLaunch e = elem_launch(q, B.Ns, TV.T);
     int rc;
-    const int ns = elem_slices(B.Ns, TV.T), blocks = elem_blocks(B.Ns, ns);
+    if (!e.threads) return QS_ERR_UNSUPPORTED;
     if (q->sbytes == 4) {
         auto k = csr_count_kernel<uint32_t, T>;
-        if ((rc = set_smem(k, sm))) return rc;
-        k<<<blocks, 32 * ELEM_WARPS, sm, st>>>(make_view<uint32_t>(q), q->staged(), B, TV, ns, rowcnt,
+        if ((rc = set_smem(k, e.smem))) return rc;
+        k<<<e.blocks, e.threads, e.smem, st>>>(make_view<uint32_t>(q), q->staged(), B, TV, e.slices, rowcnt,
                                                           flags, d_err);
     } else {
         auto k = csr_count_kernel<uint64_t, T>;
-        if ((rc = set_smem(k, sm))) return rc;
-        k<<<blocks, 32 * ELEM_WARPS, sm, st>>>(make_view<uint64_t>(q), q->staged(), B, TV, ns, rowcnt,
+        if ((rc = set_smem(k, e.smem))) return rc;
+        k<<<e.blocks, e.threads, e.smem, st>>>(make_view<uint64_t>(q), q->staged(), B, TV, e.slices, rowcnt,
                                                           flags, d_err);
     }
     QS_CHECK(cudaGetLastError());
@@ -1385,18 +1438,18 @@ template <typename T>
 static int csr_fill_t(const QsSym *q, const BasisView &B, const TermView &TV, const int64_t *rowptr, int64_t *cursor,
                       uint64_t *keys, void *vals, int *d_err, cudaStream_t st)
 {
-    size_t sm = sym_smem(q);
+    const ElemLaunch e = elem_launch(q, B.Ns, TV.T);
     int rc;
-    const int ns = elem_slices(B.Ns, TV.T), blocks = elem_blocks(B.Ns, ns);
+    if (!e.threads) return QS_ERR_UNSUPPORTED;
     if (q->sbytes == 4) {
         auto k = csr_fill_kernel<uint32_t, T>;
-        if ((rc = set_smem(k, sm))) return rc;
-        k<<<blocks, 32 * ELEM_WARPS, sm, st>>>(make_view<uint32_t>(q), q->staged(), B, TV, ns, rowptr,
+        if ((rc = set_smem(k, e.smem))) return rc;
+        k<<<e.blocks, e.threads, e.smem, st>>>(make_view<uint32_t>(q), q->staged(), B, TV, e.slices, rowptr,
                                                           cursor, keys, (T *)vals, d_err);
     } else {
         auto k = csr_fill_kernel<uint64_t, T>;
-        if ((rc = set_smem(k, sm))) return rc;
-        k<<<blocks, 32 * ELEM_WARPS, sm, st>>>(make_view<uint64_t>(q), q->staged(), B, TV, ns, rowptr,
+        if ((rc = set_smem(k, e.smem))) return rc;
+        k<<<e.blocks, e.threads, e.smem, st>>>(make_view<uint64_t>(q), q->staged(), B, TV, e.slices, rowptr,
                                                           cursor, keys, (T *)vals, d_err);
     }
     QS_CHECK(cudaGetLastError());
@@ -1554,9 +1607,9 @@ inplace_kernel(const __grid_constant__ SymParams<S> P, size_t tab_elems, BasisVi
                double ar, double ai, const cdbl *__restrict__ vin, cdbl *__restrict__ vout, int64_t nvec,
                int *__restrict__ d_err)
 {
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ ElemQueue<S> queue[ELEM_WARPS];
-    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ElemQueue<S> *queue = reinterpret_cast<ElemQueue<S> *>(smem_raw);
+    const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(queue + (blockDim.x >> 5)), tab_elems);
     int err = 0;
     for_elements(V, B, TV, nslice, queue[threadIdx.x >> 5], err,
                  [&](int, int64_t i, int64_t j, double r, double im) {
@@ -1584,18 +1637,18 @@ extern "C" int qs_inplace_op(void *sym, const void *states, const uint32_t *norm
     BasisView B{states, norms, Ns, N_p, begin, end};
     TermView TV = make_terms(t_nop, t_off, t_chr, t_site, t_J, T);
     cudaStream_t st = qs_stream(stream);
-    size_t sm = sym_smem(q);
-    const int ns = elem_slices(Ns, T), blocks = elem_blocks(Ns, ns);
+    const ElemLaunch e = elem_launch(q, Ns, T);
     int rc;
+    if (!e.threads) return QS_ERR_UNSUPPORTED;
     if (q->sbytes == 4) {
         auto k = inplace_kernel<uint32_t>;
-        if ((rc = set_smem(k, sm))) return rc;
-        k<<<blocks, 32 * ELEM_WARPS, sm, st>>>(make_view<uint32_t>(q), q->staged(), B, TV, ns, transposed, conjugated, a_re, a_im, (const cdbl *)v_in,
+        if ((rc = set_smem(k, e.smem))) return rc;
+        k<<<e.blocks, e.threads, e.smem, st>>>(make_view<uint32_t>(q), q->staged(), B, TV, e.slices, transposed, conjugated, a_re, a_im, (const cdbl *)v_in,
                                                           (cdbl *)v_out, nvec, d_err);
     } else {
         auto k = inplace_kernel<uint64_t>;
-        if ((rc = set_smem(k, sm))) return rc;
-        k<<<blocks, 32 * ELEM_WARPS, sm, st>>>(make_view<uint64_t>(q), q->staged(), B, TV, ns, transposed, conjugated, a_re, a_im, (const cdbl *)v_in,
+        if ((rc = set_smem(k, e.smem))) return rc;
+        k<<<e.blocks, e.threads, e.smem, st>>>(make_view<uint64_t>(q), q->staged(), B, TV, e.slices, transposed, conjugated, a_re, a_im, (const cdbl *)v_in,
                                                           (cdbl *)v_out, nvec, d_err);
     }
     QS_CHECK(cudaGetLastError());
@@ -1706,7 +1759,7 @@ __global__ void proj_kernel(const __grid_constant__ SymParams<S> P, size_t tab_e
                             BasisView Pc, int mode, int64_t *__restrict__ colptr, int64_t *__restrict__ rows,
                             double *__restrict__ vals, int *__restrict__ d_err)
 {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const SymView<S> V = stage_tables(P, reinterpret_cast<S *>(smem_raw), tab_elems);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const size_t tab_bytes = (tab_elems * sizeof(S) + 15) & ~(size_t)15;
@@ -1804,7 +1857,9 @@ static int proj_layout(const QsSym *q, int gsize, int &gpow2, int &wpb, size_t &
     wpb = 4;
     while (wpb > 1 && (size_t)wpb * gpow2 * (q->sbytes + 4) > 96 * 1024) wpb >>= 1;
     smem = ((q->staged_bytes() + 15) & ~(size_t)15) + (size_t)wpb * gpow2 * (q->sbytes + 4);
-    return smem > 200 * 1024 ? QS_ERR_UNSUPPORTED : QS_OK;
+    // the sign factors (lut_off - pair_off elements) ride on top of the bound
+    const size_t signs = (q->lut_off - q->pair_off) * (size_t)q->sbytes;
+    return smem > 200 * 1024 + signs ? QS_ERR_UNSUPPORTED : QS_OK;
 }
 
 // Entries of the projector, column by column (CSC).  gsize = |G| (product
