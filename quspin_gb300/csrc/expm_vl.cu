@@ -36,7 +36,7 @@ template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
 __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices,
                                         const DV *__restrict__ data, const typename M::BE *__restrict__ Bin,
                                         typename M::BE *__restrict__ Bout, cdbl *__restrict__ F, int64_t nvec,
-                                        int VL, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,
+                                        int VL, int parts, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,
                                         const cdbl *__restrict__ coeff, int j, double tol, void *ctlp)
 {
     using S = typename M::S;
@@ -89,27 +89,28 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
     }
     __syncthreads();
 
-    // 32 / VL rows per warp and sweep
-    const int RPW = 32 / VL, grp = (threadIdx.x & 31) / VL, lane0 = grp * VL, v = (threadIdx.x & 31) - lane0;
+    const int split = MULTI ? 1 : parts;
+    const VlPlace at = vl_place(VL, split);
+    const int v = at.v;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const S cf_re = s_cf[0], cf_im = s_cf[1];
     double mb = 0.0, mf = 0.0;
-    for (int64_t rb = warp * RPW; rb < n; rb += nwarps * RPW) {
-        const int64_t r = rb + grp;
+    for (int64_t rb = warp * at.rows; rb < n; rb += nwarps * at.rows) {
+        const int64_t r = rb + at.grp;
         int sec = 0;
         if constexpr (MULTI) sec = r < n ? sector_of(s_off, nsec, r) : 0;
-        const bool valid = r < n && grp < RPW && !s_done[sec];
+        const bool valid = r < n && at.grp < at.rows && !s_done[sec];
         const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
         const int bexp = s_bexp[sec];
         const S cm_re = s_cm[2 * sec], cm_im = s_cm[2 * sec + 1];
         pf rbp{0.f, 0.f}, rfp{0.f, 0.f};
         for (int64_t c0 = 0; c0 < nvec; c0 += VL) {
             const int64_t c = c0 + v < nvec ? c0 + v : nvec - 1;
-            const bool act = valid && c0 + v < nvec;
+            const bool act = valid && at.part == 0 && c0 + v < nvec;
             S ar = M::zero(), ai = M::zero();
             vl_row_sum<M, DV, true, IT, VMODE, WPL>(indices, data, codes, s_tab, Bin + c,
-                                                    (uint32_t)(nvec * sizeof(BE)), v, lane0, grp < RPW, k0, k1, ar, ai);
+                                                    (uint32_t)(nvec * sizeof(BE)), at, VL, split, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
                 const BE bo = M::ldB(Bin + e);
@@ -140,7 +141,7 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
                 rfp = pf_add(rfp, tf);
             }
         }
-        if (valid && v == 0) {
+        if (valid && at.part == 0 && v == 0) {
             const double rbn = pf_to_double_scaled(rbp, 0), rfn = pf_to_double_scaled(rfp, 0);
             if constexpr (MULTI) {
                 atomicMax(&s_mb[sec], (unsigned long long)__double_as_longlong(rbn));
@@ -204,9 +205,9 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
 #define VL_PARAMS                                                                                             \
     int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices, const DV *__restrict__ data, \
         const typename M::BE *__restrict__ Bin, typename M::BE *__restrict__ Bout, cdbl *__restrict__ F,         \
-        int64_t nvec, int VL, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,              \
+        int64_t nvec, int VL, int split, cdbl mu0, const cdbl *__restrict__ mus, const int64_t *__restrict__ sec_off,              \
         const cdbl *__restrict__ coeff, int j, double tol, void *ctlp
-#define VL_ARGS n, indptr, indices, data, Bin, Bout, F, nvec, VL, mu0, mus, sec_off, coeff, j, tol, ctlp
+#define VL_ARGS n, indptr, indices, data, Bin, Bout, F, nvec, VL, split, mu0, mus, sec_off, coeff, j, tol, ctlp
 
 template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
 __global__ void __launch_bounds__(256, 3) taylor_vl_kernel(VL_PARAMS)
@@ -220,11 +221,11 @@ int vl_go(const LpTerm &a)
     using BE = typename M::BE;
     static int resident = 0;
     auto k = taylor_vl_kernel<M, DV, IT, WPL, MULTI, VMODE>;
-    const int VL = vl_lanes(a.nvec);
-    const int64_t rows = 8 * (32 / VL);       // per block and sweep
+    const int VL = vl_lanes(a.nvec), split = MULTI ? 1 : vl_split(a.n, a.nnz, VL);
+    const int64_t rows = 8 * (32 / (VL * split));       // per block and sweep
     const int blocks = qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident);
     k<<<blocks, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, (const BE *)a.Bin,
-                                (BE *)a.Bout, a.F, a.nvec, VL, a.mu0, a.mus, a.sec_off, a.coeff, a.j, a.tol, a.ctl);
+                                (BE *)a.Bout, a.F, a.nvec, VL, split, a.mu0, a.mus, a.sec_off, a.coeff, a.j, a.tol, a.ctl);
     QS_CHECK(cudaGetLastError());
     return QS_OK;
 }

@@ -55,27 +55,62 @@ __device__ __forceinline__ void rmul_acc(typename M::S &ar, typename M::S &ai, c
     M::fma(ai, d.im, x);
 }
 
-// Lane groups of the many-vector kernels: VL lanes own a row, 32 / VL rows to
-// a warp; lanes left over own none.  The vectors are swept at most eight at a
-// time in sweeps of equal width, so few lanes go without one (13 vectors: two
-// sweeps of 7).
+// Lane groups of the many-vector kernels: VL lanes walk a row, or one of
+// `split` interleaved parts of a long one; 32 / (VL split) rows to a warp;
+// lanes left over own none.  The vectors are swept at most eight at a time in
+// sweeps of equal width, so few lanes go without one (13 vectors: two sweeps
+// of 7).
 static inline int vl_lanes(int64_t nvec)
 {
     const int64_t sweeps = (nvec + 7) / 8;
     return (int)((nvec + sweeps - 1) / sweeps);
 }
 
+// Parts of a row: a power of two that fits a warp.  Two reasons to divide it.
+// Few vectors: 16 rows to a warp read 16 far places of the words at once, so two
+// vectors take a part per 32 entries, three to five two parts from 64 or 128
+// entries (a float-pair product of 2 vectors, 60 k rows of 128 entries: 66 us in
+// one part, 50 in four; a term 64 and 49).  Few rows: parts of at least 16
+// entries while there are less than `lanes` lanes at work (8 vectors, 1000 rows
+// of 1000 entries: a product 109 -> 40 us, a term 97 -> 34; 300 rows of 300, 36
+// -> 18).  Beyond either it costs: at 60 k rows of 64 entries and 8 vectors a term
+// takes 67 us in one part, 81 in two.
+static inline int vl_split(int64_t n, int64_t nnz, int VL, int64_t lanes = 100000)
+{
+    const int64_t avg = n > 0 ? nnz / n : 0;
+    int s = 1;
+    while (2 * s * VL <= 32) {
+        const bool longs = VL == 2 ? avg >= 64 * s : VL <= 5 && s == 1 && avg >= (VL == 3 ? 64 : 128);
+        if (!longs && !(avg >= 32 * s && 2 * s * VL * n <= lanes)) break;
+        s *= 2;
+    }
+    return s;
+}
+
 constexpr int VB = 4;      // nonzeros of a row in flight
+
+// A lane's place in its warp: vector v of part `part` of row `grp` of `rows`;
+// lane0: the first lane of its VL.
+struct VlPlace {
+    int rows, grp, part, v, lane0;
+};
+__device__ __forceinline__ VlPlace vl_place(int VL, int split)
+{
+    const int lane = threadIdx.x & 31, per = VL * split, grp = lane / per, in = lane - grp * per;
+    const int part = split == 1 ? 0 : in / VL;
+    const int v = in - part * VL;
+    return {32 / per, grp, part, v, lane - v};
+}
 
 // One batch of VB nonzeros of a row for one vector, the column words in cur
 // (WPL per lane of the group, whose first lane is lane0), entry k the first.
 // FULL: all of them belong to the row; otherwise only the first `left`.  A
 // word past the row's end is zero and its gather reads column 0: an address
 // without a predicate, its product is skipped.
-template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool FULL>
+template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool FULL, class ST>
 __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, const DV *__restrict__ data,
                                          const uint8_t *__restrict__ codes, const DV *tab,
-                                         const char *__restrict__ x, uint32_t stride, IT k, int left,
+                                         const char *__restrict__ x, ST stride, IT k, int left,
                                          typename M::S (&ar)[2], typename M::S (&ai)[2])
 {
     using XE = typename std::conditional<XC, typename M::BE, typename M::S>::type;
@@ -110,44 +145,54 @@ __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, 
 // the warp fills run without predicates, addresses are one 32 x 32
 // multiply-add, and lanes past the last vector (c clamped by the caller) load
 // and compute like the rest.  Every lane of the warp calls it with its row's
-// range (empty for none; owns: the lane belongs to a row group).  x: the vectors' base at vector c; stride: bytes per
-// row of vectors.  VMODE: 0 one value per nonzero, 1 coded, 2 codes packed into
-// the column words (tab: the 256 values).
-template <class M, class DV, bool XC, class IT, int VMODE, int WPL>
+// range (empty for none).  Parts of a row take every split-th batch of it; the
+// whole sum is in part 0.  x: the vectors' base at vector c; stride: bytes per
+// row of vectors (64 bits where they pass 4 GB).  VMODE: 0 one value per
+// nonzero, 1 coded, 2 codes packed into the column words (tab: the 256 values).
+template <class M, class DV, bool XC, class IT, int VMODE, int WPL, class ST>
 __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, const DV *__restrict__ data,
                                            const uint8_t *__restrict__ codes, const DV *tab, const void *x,
-                                           uint32_t stride, int v, int lane0, bool owns, IT k0, IT k1,
+                                           ST stride, const VlPlace &at, int VL, int split, IT k0, IT k1,
                                            typename M::S &sr, typename M::S &si)
 {
-    const int len = (int)(k1 - k0);
-    const int most = __reduce_max_sync(0xffffffffu, len);
-    const int least = __reduce_min_sync(0xffffffffu, owns ? len : most);     // of the lanes that own a row
+    int len = (int)(k1 - k0);
+    const int most = __reduce_max_sync(0xffffffffu, len), step = split * VB;
+    const int least = __reduce_min_sync(0xffffffffu, at.grp < at.rows ? len : most);   // of the lanes that own a row
     const char *xb = reinterpret_cast<const char *>(x);
+    const int v = at.v, lane0 = at.lane0;
     const bool loads = v * WPL < VB;           // the lanes that fetch the words
+    // this part's first batch; a lane without a row stays below `least` in a full batch
+    k0 += (IT)(at.part * VB);
+    len -= at.part * VB;
     uint32_t word[WPL];
     auto fetch = [&](int b) {
 #pragma unroll
         for (int i = 0; i < WPL; i++) {
-            const int at = b + v * WPL + i;
-            word[i] = loads && at < len ? (uint32_t)__ldcs(indices + k0 + at) : 0u;
+            const int k = b + v * WPL + i;
+            word[i] = loads && k < len ? (uint32_t)__ldcs(indices + k0 + k) : 0u;
         }
     };
     // even and odd places apart, as two lanes of a row hand-out: half the
     // roundings that one chain collects
     typename M::S ar[2] = {M::zero(), M::zero()}, ai[2] = {M::zero(), M::zero()};
     fetch(0);
-    for (int b = 0; b < most; b += VB) {
+    for (int b = 0; b < most; b += step) {
         uint32_t cur[WPL];
 #pragma unroll
         for (int i = 0; i < WPL; i++) cur[i] = word[i];
-        fetch(b + VB);
-        if (b + VB <= least)
+        fetch(b + step);
+        if (b + step <= least)
             vl_batch<M, DV, XC, IT, VMODE, WPL, true>(cur, lane0, data, codes, tab, xb, stride, k0 + b, VB, ar, ai);
         else
             vl_batch<M, DV, XC, IT, VMODE, WPL, false>(cur, lane0, data, codes, tab, xb, stride, k0 + b, len - b, ar, ai);
     }
     sr = M::merge(ar[0], ar[1]);
     si = M::merge(ai[0], ai[1]);
+    for (int o = 1; o < split; o <<= 1) {
+        const int from = (threadIdx.x & 31) + o * VL;
+        sr = M::merge(sr, M::shfl(sr, from));
+        si = M::merge(si, M::shfl(si, from));
+    }
 }
 
 }  // namespace

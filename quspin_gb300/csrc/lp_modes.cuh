@@ -62,6 +62,10 @@ struct ModePF {
     {
         return pf{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
     }
+    __device__ static S shfl(S a, int src)
+    {
+        return pf{__shfl_sync(0xffffffffu, a.h, src & 31), __shfl_sync(0xffffffffu, a.l, src & 31)};
+    }
     __device__ static S ldS(const S *p)
     {
         const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
@@ -105,6 +109,7 @@ struct ModeF32 {
     __device__ static float hi(S a) { return a; }
     __device__ static S from_d(double x) { return (float)x; }
     __device__ static S shfl_xor(S a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+    __device__ static S shfl(S a, int src) { return __shfl_sync(0xffffffffu, a, src & 31); }
     __device__ static S ldS(const S *p) { return __ldg(p); }
     __device__ static double add_to(double f, S v, int k) { return f + f2d_scaled(v, k); }
     __device__ static double to_d(S v, int k) { return f2d_scaled(v, k); }

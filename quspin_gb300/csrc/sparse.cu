@@ -235,7 +235,7 @@ static int spmm_idx(int idx64, int64_t n, const void *indptr, const int32_t *ind
 // precision never exceeds the vector precision's partner).  group: launch
 // shape, G | (U << 8) with G lanes per row (2..32) and U in-flight entries per
 // lane (1, 2, 4); 0 picks G from nnz/n and U = 2.
-int spmv_lp_single(int64_t n, const void *indptr, int idx64, const int32_t *indices, const void *data, int dtype,
+int spmv_lp_single(int64_t n, int64_t nnz, const void *indptr, int idx64, const int32_t *indices, const void *data, int dtype,
                    const void *x, int xtype, void *y, int64_t nvec, cdbl a, int overwrite, int G, int U,
                    cudaStream_t st);
 
@@ -261,7 +261,7 @@ extern "C" int qs_csr_matvec(int64_t n, int64_t nnz, const void *indptr, int idx
         return QS_ERR_ARG;
     case QS_F32:
         if (dtype == QS_F32)   // FP32 products and row sums (csrc/spmv_lp.cu)
-            return spmv_lp_single(n, indptr, idx64, indices, data, dtype, x, xtype, y, nvec, a, overwrite, G, U, st);
+            return spmv_lp_single(n, nnz, indptr, idx64, indices, data, dtype, x, xtype, y, nvec, a, overwrite, G, U, st);
         return QS_ERR_ARG;
     case QS_C128:
         if (dtype == QS_F64) return spmm_idx<double, cdbl>(idx64, n, indptr, indices, data, x, y, nvec, a, overwrite, G, U, st);
@@ -271,7 +271,7 @@ extern "C" int qs_csr_matvec(int64_t n, int64_t nnz, const void *indptr, int idx
         return QS_ERR_ARG;
     case QS_C64:
         if (dtype == QS_F32 || dtype == QS_C64)
-            return spmv_lp_single(n, indptr, idx64, indices, data, dtype, x, xtype, y, nvec, a, overwrite, G, U, st);
+            return spmv_lp_single(n, nnz, indptr, idx64, indices, data, dtype, x, xtype, y, nvec, a, overwrite, G, U, st);
         return QS_ERR_ARG;
     default:
         return QS_ERR_ARG;

@@ -230,11 +230,11 @@ __global__ void __launch_bounds__(256) spmv_lz_kernel(LzProduct p, int lgG)
 // 194 us then, 120 us now; 5 vectors 112 / 87 us; J1-J2 L = 28 (361 k rows,
 // 10.7 M real nonzeros): 8 vectors 401 / 191 us, 2 vectors 98 / 69 us.  Complex
 // pairs run at three blocks per SM (four spill: 129 us), the rest at four.
-template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL>
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST>
 __global__ void __launch_bounds__(256, std::is_same<DV, cpf>::value ? 3 : 4)
 spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices,
                const DV *__restrict__ data, const void *__restrict__ xv, YT *__restrict__ y, int64_t nvec, int VL,
-               cdbl a, int overwrite, const unsigned long long *__restrict__ xnorm)
+               int split, cdbl a, int overwrite, const unsigned long long *__restrict__ xnorm)
 {
     using S = typename M::S;
     using XE = typename std::conditional<XC, typename M::BE, S>::type;
@@ -254,19 +254,21 @@ spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restri
     __syncthreads();
     const cx<S> av{s_a[0], s_a[1]};
     const int k2 = s_k;
-    const int RPW = 32 / VL, grp = (threadIdx.x & 31) / VL, lane0 = grp * VL, v = (threadIdx.x & 31) - lane0;
+    const VlPlace at = vl_place(VL, split);
+    const int v = at.v;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t rb = warp * RPW; rb < n; rb += nwarps * RPW) {
-        const int64_t r = rb + grp;
-        const bool valid = r < n && grp < RPW;
+    for (int64_t rb = warp * at.rows; rb < n; rb += nwarps * at.rows) {
+        const int64_t r = rb + at.grp;
+        const bool valid = r < n && at.grp < at.rows;
         const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
-        for (int64_t c0 = 0; c0 < nvec; c0 += VL) {
+        // all sweeps, or one of them for each gridDim.y
+        for (int64_t c0 = (int64_t)blockIdx.y * VL; c0 < nvec; c0 += (int64_t)gridDim.y * VL) {
             const int64_t c = c0 + v < nvec ? c0 + v : nvec - 1;
-            const bool act = valid && c0 + v < nvec;
+            const bool act = valid && at.part == 0 && c0 + v < nvec;
             S ar = M::zero(), ai = M::zero();
             vl_row_sum<M, DV, XC, IT, VM, WPL>(indices, data, codes, s_tab, reinterpret_cast<const XE *>(xv) + c,
-                                               (uint32_t)(nvec * sizeof(XE)), v, lane0, grp < RPW, k0, k1, ar, ai);
+                                               (ST)(nvec * sizeof(XE)), at, VL, split, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
                 const S accr = M::fin(ar);
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(256) xsplit_kernel(int64_t count, const double
 }
 
 struct SpmvArgs {
-    int64_t n;
+    int64_t n, nnz;
     const void *indptr;
     int idx64;
     const int32_t *indices;
@@ -362,16 +364,22 @@ int spmv_go(const SpmvArgs &a)
     return QS_OK;
 }
 
-template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL>
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST = uint32_t>
 int spmm_go(const SpmvArgs &a)
 {
     static int resident = 0;
-    auto k = spmm_vl_kernel<M, DV, XC, YT, IT, VM, WPL>;
-    const int VL = vl_lanes(a.nvec);
-    const int64_t rows = 8 * (32 / VL);       // per block and sweep
-    const int blocks = qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident);
-    k<<<blocks, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, a.x, (YT *)a.y, a.nvec, VL,
-                                a.a, a.overwrite, a.xnorm);
+    auto k = spmm_vl_kernel<M, DV, XC, YT, IT, VM, WPL, ST>;
+    // FP32 arithmetic leaves more of the latency to hide than float pairs do
+    const int64_t lanes = std::is_same<M, ModeF32>::value ? 130000 : 100000;
+    const int VL = vl_lanes(a.nvec), split = vl_split(a.n, a.nnz, VL, lanes);
+    const int64_t rows = 8 * (32 / (VL * split));       // per block and sweep
+    // with few rows the sweeps go to blocks of their own, too
+    int64_t apart = lanes / (a.n * VL * split);
+    if (apart > 64) apart = 64;
+    if (apart > (a.nvec + VL - 1) / VL) apart = (a.nvec + VL - 1) / VL;
+    const dim3 grid(qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident), (unsigned)(apart < 1 ? 1 : apart));
+    k<<<grid, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, a.x, (YT *)a.y, a.nvec, VL,
+                              split, a.a, a.overwrite, a.xnorm);
     QS_CHECK(cudaGetLastError());
     return QS_OK;
 }
@@ -412,11 +420,11 @@ int spmv_idx(const SpmvArgs &a)
 
 // float32 / complex64 operands (called by qs_csr_matvec): 0 when handled,
 // QS_ERR_UNSUPPORTED for type pairs left to the double kernels.
-int spmv_lp_single(int64_t n, const void *indptr, int idx64, const int32_t *indices, const void *data, int dtype,
+int spmv_lp_single(int64_t n, int64_t nnz, const void *indptr, int idx64, const int32_t *indices, const void *data, int dtype,
                    const void *x, int xtype, void *y, int64_t nvec, cdbl a, int overwrite, int G, int U,
                    cudaStream_t st)
 {
-    SpmvArgs s{n, indptr, idx64, indices, data, x, y, nvec, a, overwrite, nullptr, G, U, st};
+    SpmvArgs s{n, nnz, indptr, idx64, indices, data, x, y, nvec, a, overwrite, nullptr, G, U, st};
     if (xtype == QS_F32 && dtype == QS_F32) return spmv_idx<ModeF32, float, false, float>(s);
     if (xtype == QS_C64 && dtype == QS_F32) return spmv_idx<ModeF32, float, true, cflt>(s);
     if (xtype == QS_C64 && dtype == QS_C64) return spmv_idx<ModeF32, cx<float>, true, cflt>(s);
@@ -510,7 +518,7 @@ extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, i
     if (sell_type(pdtype))
         return sell_spmv(n, (const int64_t *)indptr, indices, pdata, pdtype, xs, xc, y, cdbl{a_re, a_im}, overwrite, nrm,
                          st);
-    SpmvArgs s{n, indptr, idx64, indices, pdata, xs, y, nvec, cdbl{a_re, a_im}, overwrite, nrm, G, U, st};
+    SpmvArgs s{n, nnz, indptr, idx64, indices, pdata, xs, y, nvec, cdbl{a_re, a_im}, overwrite, nrm, G, U, st};
     if (pdtype == QS_PF8) return xc ? spmv_idx<ModePF, pf, true, cdbl, 1>(s) : spmv_idx<ModePF, pf, false, double, 1>(s);
     if (pdtype == QS_CPF8) return spmv_idx<ModePF, cpf, true, cdbl, 1>(s);
     const bool v4 = ((group >> 20) & 7) == 6 && group > 0;
