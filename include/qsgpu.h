@@ -201,7 +201,8 @@ int qs_sell_count(int64_t n, const int32_t *d_indptr, int64_t *d_groups, int *d_
 int qs_sell_fill(int64_t n, const int32_t *d_indptr, const int32_t *d_words, const int64_t *d_sptr, int64_t groups,
                  int32_t *d_out, void *stream);
 /* The same for one vector in float-pair storage on a small int32 matrix (at
- * most 2^17 rows; dtype 4 / 5, or coded 6 / 7) as one cooperative launch.
+ * most 2^17 rows and 2^30 entries; dtype 4 / 5, or coded 6 / 7) as one
+ * cooperative launch.
  * d_sync: qs_expm_small_sync_bytes() of zeros before the first call; calls
  * that share d_work, d_ctl or d_sync must not overlap. */
 int qs_expm_small_sync_bytes(void);

@@ -18,8 +18,8 @@
 // (245 rows, 27 terms of 35) 274 -> 137 us; XXZ L = 20 (4752 rows, 54 of 80)
 // 661 -> 285; Ising L = 18 (14541 rows, 274k nonzeros, 117 of 165) 1534 -> 908;
 // Ising L = 20 (52377 rows, 1.1M nonzeros, 126 of 165) 2262 -> 1828.  Above
-// 65535 rows the launch shapes of csrc/expm_lp.cu are tuned and its resident
-// warps hide the gathers better than one block per SM.  The rows on 128, 76 or
+// 65535 rows, and 2.4 M entries, the launch shapes of csrc/expm_lp.cu are tuned or
+// its resident warps hide the gathers better than one block per SM.  The rows on 128, 76 or
 // 38 SMs instead of all 152: 294, 310, 385 us at 4752 rows, and more above.
 //
 // B changes hands between SMs inside the kernel: it is written through to L2
@@ -308,7 +308,8 @@ int small_go(SmallArgs p, int64_t nnz, cudaStream_t st)
 extern "C" int qs_expm_small_sync_bytes() { return (int)sizeof(SmallSync); }
 
 // qs_expm_multiply for one vector and float-pair storage (btype QS_CPF) of a
-// small int32 matrix, as one cooperative launch: at most 2^17 rows; dtype
+// small int32 matrix, as one cooperative launch: at most 2^17 rows and 2^30
+// entries (an entry index and the lanes' stride fit an int); dtype
 // QS_PF / QS_CPF or coded QS_PF8 / QS_CPF8.  sync: qs_expm_small_sync_bytes()
 // of zeros before the first call, left zero; calls that share ctl, work or
 // sync must not overlap.  The control block receives this call's terms and
@@ -319,7 +320,7 @@ extern "C" int qs_expm_multiply_small(int64_t n, int64_t nnz, const int32_t *ind
                                       double mu_re, double mu_im, const void *coeff, const void *eta, void *work,
                                       void *ctl, void *sync, void *stream)
 {
-    if (n < 1 || n > (1 << 17) || nnz < 0 || s < 1 || m_star < 0 || !indptr || !F || !coeff || !eta || !work || !ctl ||
+    if (n < 1 || n > (1 << 17) || nnz < 0 || nnz > (1 << 30) || s < 1 || m_star < 0 || !indptr || !F || !coeff || !eta || !work || !ctl ||
         !sync || (nnz > 0 && (!indices || !data)))
         return QS_ERR_ARG;
     SmallArgs p{(int)n, 1, s, m_star, indptr, indices, data, (cpf *)work, (cpf *)work + n, (cdbl *)F,

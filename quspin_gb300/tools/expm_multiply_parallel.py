@@ -303,15 +303,20 @@ class ExpmMultiplyParallel:
     # largest problem evolved in one cooperative launch (csrc/expm_small.cu):
     # below the sizes whose launch shapes are tuned.  Against the graph of one
     # launch per term: 137 against 274 us at 245 rows, 285 against 661 at 4752,
-    # 1828 against 2262 at 52377
+    # 1828 against 2262 at 52377.  Rows of many entries gain less, their gathers
+    # being most of a term, and past some 2.5 M entries the other kernels' greater
+    # number of warps wins: 40 k rows of 64 324 against 291 us, 20 k of 300 489 /
+    # 373, 60 k of 300 1005 / 770; below, 60 k of 40 219 / 289, 1500 of 1500 203 / 218
     SMALL_MAX_ROWS = 65535
+    SMALL_MAX_NNZ = 2_400_000
 
     def _small_operand(self):
         """The coded or plain float-pair operand of the one-launch evolution,
         or None where it does not apply (other precisions, larger or int64
         matrices, a launch shape set by hand)."""
         A = self._Ad
-        if self._precision != "double" or A.idx64 or not 0 < A.shape[0] <= self.SMALL_MAX_ROWS:
+        if (self._precision != "double" or A.idx64 or not 0 < A.shape[0] <= self.SMALL_MAX_ROWS
+                or A.nnz > self.SMALL_MAX_NNZ):
             return None
         from ..tune import tune_taylor
         P, btype = self._operand(1)

@@ -82,3 +82,14 @@ def test_binding_argument_counts_and_kinds_match_header():
                 assert a is ctypes.c_double, (name, p)
             elif p.startswith("int"):
                 assert a is ctypes.c_int, (name, p)
+
+
+def test_small_evolution_refuses_what_its_indices_do_not_hold():
+    """The one-launch evolution walks its entries with ints: it takes 2^30 and
+    refuses more before it looks at any pointer."""
+    L = _lib()
+    lib = L.load()
+    args = lambda n, nnz, indices: (n, nnz, 1, indices, 1, L.PF, 1, 1, 5, 1e-16, 0.0, 0.0, 1, 1, 1, 1, 1, None)
+    assert lib.qs_expm_multiply_small(*args(1000, (1 << 30) + 1, 1)) == -1
+    assert lib.qs_expm_multiply_small(*args(1000, 2**31 - 1, 1)) == -1
+    assert lib.qs_expm_multiply_small(*args((1 << 17) + 1, 10, 1)) == -1

@@ -89,3 +89,28 @@ def test_small_edges(cuda):
     assert Z.m_star == 0
     np.testing.assert_allclose(Z.dot(v), v, rtol=0, atol=0)
     assert D.to_device(v).shape == (n,)
+
+
+@pytest.mark.parametrize("row,one", [(39, True), (41, False)])
+def test_small_form_by_entries(cuda, row, one):
+    """Many entries in few rows go to the launch per term: its rule counts
+    both, and the two agree."""
+    from quspin_gb300 import _device as D
+    from quspin_gb300.sparse import DeviceCSR
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    n = 60000
+    rng = np.random.default_rng(row)
+    cols = (np.arange(n)[:, None] + rng.choice(n, row, replace=False)[None, :]) % n
+    A = sp.csr_matrix((rng.choice(np.array([0.5, -1.0, 0.25]), n * row) / row, np.sort(cols, axis=1).ravel(),
+                       np.arange(n + 1) * row), shape=(n, n))
+    op = ExpmMultiplyParallel(DeviceCSR.from_scipy(A), a=-0.5j)
+    assert (op._small_operand() is not None) == one
+    v = rng.normal(size=n) + 1j * rng.normal(size=n)
+    got = op.dot(D.to_device(v))
+    old = ExpmMultiplyParallel.SMALL_MAX_NNZ
+    ExpmMultiplyParallel.SMALL_MAX_NNZ = 0 if one else 1 << 30
+    try:
+        ref = op.dot(D.to_device(v))
+    finally:
+        ExpmMultiplyParallel.SMALL_MAX_NNZ = old
+    assert float((got - ref).norm() / ref.norm()) <= 1e-13
