@@ -204,8 +204,15 @@ int qs_sell_fill(int64_t n, const int32_t *d_indptr, const int32_t *d_words, con
  * most 2^17 rows and 2^30 entries; dtype 4 / 5, or coded 6 / 7) as one
  * cooperative launch.
  * d_sync: qs_expm_small_sync_bytes() of zeros before the first call; calls
- * that share d_work, d_ctl or d_sync must not overlap. */
+ * that share d_work, d_ctl or d_sync must not overlap.  A grid barrier gives up
+ * after qs_expm_small_polls() looks, or `polls` of them: d_F is NaN then and the
+ * 13th int of d_ctl is nonzero.  d_keep (n elements, or NULL) receives the input. */
 int qs_expm_small_sync_bytes(void);
+int qs_expm_small_polls(void);
+int qs_expm_multiply_small_kept(int64_t n, int64_t nnz, const int32_t *d_indptr, const int32_t *d_indices,
+                                const void *d_data, int dtype, void *d_F, int s, int m_star, double tol, double mu_re,
+                                double mu_im, const void *d_coeff, const void *d_eta, void *d_work, void *d_ctl,
+                                void *d_sync, void *d_keep, int polls, void *stream);
 int qs_expm_multiply_small(int64_t n, int64_t nnz, const int32_t *d_indptr, const int32_t *d_indices,
                            const void *d_data, int dtype, void *d_F, int s, int m_star, double tol, double mu_re,
                            double mu_im, const void *d_coeff, const void *d_eta, void *d_work, void *d_ctl,

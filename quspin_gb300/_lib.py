@@ -73,6 +73,9 @@ _SIGS = {
     "qs_csr_trace": (_i, [_i64, _vp, _i, _vp, _vp, _i, _vp, _vp, _vp]),
     "qs_csr_1_norm": (_i, [_i64, _vp, _i, _vp, _vp, _i, _d, _d, _vp, _vp, _vp, _vp]),
     "qs_expm_small_sync_bytes": (_i, []),
+    "qs_expm_small_polls": (_i, []),
+    "qs_expm_multiply_small_kept": (_i, [_i64, _i64, _vp, _vp, _vp, _i, _vp, _i, _i, _d, _d, _d, _vp, _vp, _vp, _vp, _vp,
+                                         _vp, _i, _vp]),
     "qs_value_codes_state_bytes": (_i, []),
     "qs_value_codes": (_i, [_i64, _vp, _i, _vp, _vp, _vp, _vp]),
     "qs_sell_count": (_i, [_i64, _vp, _vp, _vp, _vp]),

@@ -12,7 +12,7 @@ struct ExpmCtl {
     long long terms;           // Taylor terms executed so far
     int nonconv;               // substeps that used all m* terms without the test firing
     int bexp;                  // B is stored scaled by 2^-bexp (paired / single-precision storage)
-    int err;                   // nonzero: a bounded device wait gave up (staged term kernel)
+    int err;                   // nonzero: a bounded device wait gave up (csrc/expm_small.cu)
     int pad_;
 };
 

@@ -25,8 +25,10 @@
 // B changes hands between SMs inside the kernel: it is written through to L2
 // and gathered past L1 (ld.cg); the matrix is read through L1, where each SM's
 // rows stay from term to term.  The barrier counts arrivals upwards and gives
-// up after a bounded number of polls (err in the control block); the launch is
-// cooperative, so every block is resident and the wait ends.
+// up after a bounded number of polls; the launch is cooperative, so every block
+// is resident and the wait ends.  Should it give up all the same, F is NaN, err
+// is set in the control block and the input is kept for another way to evolve
+// it (ExpmMultiplyParallel.settle).
 #include "qs_common.cuh"
 #include "expm_ctl.cuh"
 #include "lp_lanes.cuh"
@@ -35,21 +37,21 @@ namespace {
 
 constexpr int CT = 512;              // most threads per block
 constexpr int CU = 4;                // gathers in flight per lane
-constexpr int POLLS = 1 << 23;       // about a second
+constexpr int POLLS = 1 << 23;       // a few seconds: a poll is a trip to L2 and back
 
 // Arrival count and the maxima of three reductions in turn; all zero between
-// launches.  left: blocks that have finished.
+// launches.  left: blocks that have finished; failed: whose wait gave up.
 struct SmallSync {
-    unsigned int arrive, left;
+    unsigned int arrive, left, failed, pad_;
     unsigned long long mb[3], mf[3];
 };
 
 struct SmallArgs {
-    int n, lgG, s, m;
+    int n, lgG, s, m, polls;
     const int32_t *indptr, *indices;
     const void *data;
     cpf *B0, *B1;
-    cdbl *F;
+    cdbl *F, *keep;            // keep: receives the input (nullable)
     const cdbl *coeff, *eta;
     cdbl mu;
     double tol;
@@ -70,10 +72,11 @@ __device__ __forceinline__ cpf ld_val(const cpf *p) { return ModePF::ldB(p); }
 __device__ __forceinline__ unsigned long long max64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
 // Grid-wide maxima of two doubles >= 0 (as bits), reduction number e, which is
-// also a barrier.  False when the wait gave up.  (Every block posting a word
+// also a barrier.  False when the wait gave up after `most` polls.  (Every block posting a word
 // that all others poll, without atomics, measured twice as slow: 149 pollers on
 // each of 149 lines.)
-__device__ __forceinline__ bool grid_max2(SmallSync *sync, unsigned &e, unsigned long long &a, unsigned long long &b)
+__device__ __forceinline__ bool grid_max2(SmallSync *sync, int most, unsigned &e, unsigned long long &a,
+                                          unsigned long long &b)
 {
     __shared__ unsigned long long sa[CT / 32], sb[CT / 32];
     __shared__ int ok;
@@ -100,9 +103,9 @@ __device__ __forceinline__ bool grid_max2(SmallSync *sync, unsigned &e, unsigned
         atomicAdd(&sync->arrive, 1u);
         const unsigned target = e * gridDim.x;
         int polls = 0;
-        while ((int)(*((volatile unsigned int *)&sync->arrive) - target) < 0 && ++polls < POLLS) {}
+        while ((int)(*((volatile unsigned int *)&sync->arrive) - target) < 0 && ++polls < most) {}
         __threadfence();
-        ok = polls < POLLS;
+        ok = polls < most;
         sa[0] = __ldcg(&sync->mb[slot]);
         sb[0] = __ldcg(&sync->mf[slot]);
     }
@@ -154,7 +157,6 @@ __global__ void __launch_bounds__(CT, 1) taylor_small_kernel(SmallArgs p)
     long long terms = 0;
     unsigned long long c1 = 0ull;       // bits of c1, or of its square after the first term
     bool ok = true;
-    if (tid == 0) p.ctl->err = 0;
     for (int step = 0; step <= p.s && ok; step++) {
         // F = eta F (not before the first substep), its norm, B0 = F 2^-bexp
         const bool scale = step > 0 && !(eta.x == 1.0 && eta.y == 0.0);
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(CT, 1) taylor_small_kernel(SmallArgs p)
         for (int r = tid; r < p.n; r += nthreads) {
             const double2 v = __ldcg(reinterpret_cast<const double2 *>(p.F + r));
             double fx = v.x, fy = v.y;
+            if (step == 0 && p.keep) __stcg(reinterpret_cast<double2 *>(p.keep + r), v);
             if (scale) {
                 fx = eta.x * v.x - eta.y * v.y;
                 fy = eta.x * v.y + eta.y * v.x;
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(CT, 1) taylor_small_kernel(SmallArgs p)
             }
         }
         if (step == p.s) break;
-        ok = grid_max2(p.sync, e, mb, mf);
+        ok = grid_max2(p.sync, p.polls, e, mb, mf);
         if (!ok) break;
         c1 = mb;
         bexp = scale_exp(__longlong_as_double((long long)c1));
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(CT, 1) taylor_small_kernel(SmallArgs p)
             __stcg(reinterpret_cast<float4 *>(p.B0 + r), make_float4(re.h, re.l, im.h, im.l));
         }
         mb = mf = 0ull;
-        ok = grid_max2(p.sync, e, mb, mf);
+        ok = grid_max2(p.sync, p.polls, e, mb, mf);
         bool done = false;
         for (int j = 0; j < p.m && ok && !done; j++) {
             const cpf *Bin = (j & 1) ? p.B1 : p.B0;
@@ -251,31 +254,37 @@ __global__ void __launch_bounds__(CT, 1) taylor_small_kernel(SmallArgs p)
                     if (f2 == f2) mf = max64(mf, (unsigned long long)__double_as_longlong(f2));
                 }
             }
-            ok = grid_max2(p.sync, e, mb, mf);
+            ok = grid_max2(p.sync, p.polls, e, mb, mf);
             done = stop_test(c1, j == 0, mb, mf, p.tol, bexp);
             if (!done) c1 = mb;
             terms++;
         }
         if (p.m > 0 && !done) nonconv++;
     }
-    if (!ok)          // a barrier gave up: no result rather than a wrong one
-        for (int r = tid; r < p.n; r += nthreads) p.F[r] = cdbl{__longlong_as_double(-1ll), __longlong_as_double(-1ll)};
-    // the last block to leave clears the words for the next launch
-    __shared__ bool last;
+    // the last block to leave clears the words for the next launch; where a
+    // barrier gave up it leaves no result rather than a wrong one
+    __shared__ bool last, failed;
     __syncthreads();
     if (threadIdx.x == 0) {
         if (blockIdx.x == 0) {
             p.ctl->terms = terms;
             p.ctl->nonconv = nonconv;
         }
-        if (!ok) p.ctl->err = 1;
+        if (!ok) atomicOr(&p.sync->failed, 1u);
         __threadfence();
         last = atomicAdd(&p.sync->left, 1u) + 1u == gridDim.x;
+        __threadfence();
+        failed = last && *((volatile unsigned int *)&p.sync->failed);
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
+    if (!last) return;
+    if (failed)
+        for (int r = threadIdx.x; r < p.n; r += blockDim.x)
+            p.F[r] = cdbl{__longlong_as_double(-1ll), __longlong_as_double(-1ll)};
+    if (threadIdx.x == 0) {
+        p.ctl->err = failed;
         for (int i = 0; i < 3; i++) p.sync->mb[i] = p.sync->mf[i] = 0ull;
-        p.sync->arrive = 0u;
+        p.sync->arrive = p.sync->failed = 0u;
         __threadfence();
         p.sync->left = 0u;
     }
@@ -314,17 +323,18 @@ extern "C" int qs_expm_small_sync_bytes() { return (int)sizeof(SmallSync); }
 // of zeros before the first call, left zero; calls that share ctl, work or
 // sync must not overlap.  The control block receives this call's terms and
 // unconverged substeps (nothing is added up), and in its err word whether a
-// grid barrier gave up; F is NaN then.
-extern "C" int qs_expm_multiply_small(int64_t n, int64_t nnz, const int32_t *indptr, const int32_t *indices,
-                                      const void *data, int dtype, void *F, int s, int m_star, double tol,
-                                      double mu_re, double mu_im, const void *coeff, const void *eta, void *work,
-                                      void *ctl, void *sync, void *stream)
+// grid barrier gave up after `polls` looks (a limit of the caller's for tests
+// and watchdogs); F is NaN then, and keep (n elements, nullable) holds the input.
+extern "C" int qs_expm_multiply_small_kept(int64_t n, int64_t nnz, const int32_t *indptr, const int32_t *indices,
+                                           const void *data, int dtype, void *F, int s, int m_star, double tol,
+                                           double mu_re, double mu_im, const void *coeff, const void *eta, void *work,
+                                           void *ctl, void *sync, void *keep, int polls, void *stream)
 {
     if (n < 1 || n > (1 << 17) || nnz < 0 || nnz > (1 << 30) || s < 1 || m_star < 0 || !indptr || !F || !coeff || !eta || !work || !ctl ||
-        !sync || (nnz > 0 && (!indices || !data)))
+        !sync || polls < 0 || polls > POLLS || (nnz > 0 && (!indices || !data)))
         return QS_ERR_ARG;
-    SmallArgs p{(int)n, 1, s, m_star, indptr, indices, data, (cpf *)work, (cpf *)work + n, (cdbl *)F,
-                (const cdbl *)coeff, (const cdbl *)eta, cdbl{mu_re, mu_im}, tol, (ExpmCtl *)ctl, (SmallSync *)sync};
+    SmallArgs p{(int)n, 1, s, m_star, polls, indptr, indices, data, (cpf *)work, (cpf *)work + n, (cdbl *)F,
+                (cdbl *)keep, (const cdbl *)coeff, (const cdbl *)eta, cdbl{mu_re, mu_im}, tol, (ExpmCtl *)ctl, (SmallSync *)sync};
     switch (dtype) {
     case QS_PF: return small_go<pf, 0>(p, nnz, qs_stream(stream));
     case QS_CPF: return small_go<cpf, 0>(p, nnz, qs_stream(stream));
@@ -332,4 +342,16 @@ extern "C" int qs_expm_multiply_small(int64_t n, int64_t nnz, const int32_t *ind
     case QS_CPF8: return small_go<cpf, 1>(p, nnz, qs_stream(stream));
     default: return QS_ERR_ARG;
     }
+}
+
+extern "C" int qs_expm_small_polls() { return POLLS; }
+
+// The same without a kept input, up to the largest number of polls.
+extern "C" int qs_expm_multiply_small(int64_t n, int64_t nnz, const int32_t *indptr, const int32_t *indices,
+                                      const void *data, int dtype, void *F, int s, int m_star, double tol,
+                                      double mu_re, double mu_im, const void *coeff, const void *eta, void *work,
+                                      void *ctl, void *sync, void *stream)
+{
+    return qs_expm_multiply_small_kept(n, nnz, indptr, indices, data, dtype, F, s, m_star, tol, mu_re, mu_im, coeff,
+                                       eta, work, ctl, sync, nullptr, POLLS, stream);
 }

@@ -270,11 +270,13 @@ class ExpmMultiplyParallel:
         """In place e^{aA} F for a complex128 device tensor F of shape (n,) or
         (n, k).  Returns F.  No host synchronisation, except with a learned
         (m*, s), where the substep counter is read once to decide on the
-        fallback to the plain selection."""
+        fallback to the plain selection.  ``settle`` makes sure of a result
+        that is not read back otherwise."""
         if self.partition_source != "learned":
             return self._run_device(F, tol, work)
         saved = F.clone()
         self._run_device(F, tol, work)
+        self.settle(F, tol)
         if self.nonconverged_substeps:
             self.fallbacks = self.__dict__.get("fallbacks", 0) + 1
             self._calculate_partition(plain=True)
@@ -282,11 +284,22 @@ class ExpmMultiplyParallel:
             self._run_device(F, tol, work)
         return F
 
-    def _run_device(self, F, tol=None, work=None):
+    def settle(self, F, tol=None):
+        """Waits for the last evolution of the device tensor F.  Where its
+        one-launch form gave up on a barrier (F is NaN then), evolves the kept
+        input again with a launch per term.  Returns F.  Host results have been
+        through this; a program that keeps its states on the device can call it
+        where it waits anyway."""
+        if self.gave_up:
+            F.view(-1).copy_(self._keep)
+            self._run_device(F, tol, one_launch=False)
+        return F
+
+    def _run_device(self, F, tol=None, work=None, one_launch=True):
         n = self._Ad.shape[0]
         nvec = 1 if F.dim() == 1 else F.shape[1]
         tol = float(self._tol if tol is None else tol)
-        if nvec == 1 and F.is_contiguous() and self._small_operand() is not None \
+        if one_launch and nvec == 1 and F.is_contiguous() and self._small_operand() is not None \
                 and not torch.cuda.is_current_stream_capturing():
             return self._run_small(F, tol)
         if (work is None and n * nvec <= self.GRAPH_MAX_ELEMS and F.is_contiguous()
@@ -309,6 +322,7 @@ class ExpmMultiplyParallel:
     # 373, 60 k of 300 1005 / 770; below, 60 k of 40 219 / 289, 1500 of 1500 203 / 218
     SMALL_MAX_ROWS = 65535
     SMALL_MAX_NNZ = 2_400_000
+    SMALL_POLLS = None      # looks after which its barriers give up (None: the library's limit, a few seconds)
 
     def _small_operand(self):
         """The coded or plain float-pair operand of the one-launch evolution,
@@ -330,15 +344,17 @@ class ExpmMultiplyParallel:
         if sync is None:
             sync = self._sync = torch.zeros(_lib.load().qs_expm_small_sync_bytes() // 8, dtype=torch.int64,
                                             device=D.device())
+            self._keep = torch.empty(n, dtype=torch.complex128, device=D.device())
         key = (complex(self._a), complex(self._mu), int(self._s), int(self._m_star))
         kept = self.__dict__.get("_small_consts")
         if kept is None or kept[0] != key:
             kept = self._small_consts = (key, self._const_table())
         consts, m = kept[1], max(int(self._m_star), 1)
         mu = complex(self._mu)
-        _lib.call("qs_expm_multiply_small", n, P.nnz, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(P.data), P.vcode,
+        polls = _lib.load().qs_expm_small_polls() if self.SMALL_POLLS is None else self.SMALL_POLLS
+        _lib.call("qs_expm_multiply_small_kept", n, P.nnz, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(P.data), P.vcode,
                   D.ptr(F), int(self._s), int(self._m_star), tol, mu.real, mu.imag, D.ptr(consts),
-                  D.ptr(consts[m:m + 1]), D.ptr(work), D.ptr(ctl), D.ptr(sync), D.stream())
+                  D.ptr(consts[m:m + 1]), D.ptr(work), D.ptr(ctl), D.ptr(sync), D.ptr(self._keep), polls, D.stream())
         self._last_ctl = ctl
         return F
 
@@ -406,19 +422,35 @@ class ExpmMultiplyParallel:
         return F
 
     @property
+    def gave_up(self):
+        """Whether the last evolution gave up on a barrier of its one-launch
+        form and left NaN (reads the device word; see ``settle``)."""
+        c = getattr(self, "_last_ctl", None)
+        return c is not None and bool(c.view(torch.int32)[12].item())
+
+    def _counters(self):
+        """The last evolution's control words as host int32; raises where it
+        gave up."""
+        c = getattr(self, "_last_ctl", None)
+        if c is None:
+            return None
+        words = c.view(torch.int32).tolist()
+        if words[12]:
+            raise _lib.QsError("the last evolution gave up on a grid barrier and left NaN: settle(F) evolves it again")
+        return words
+
+    @property
     def nonconverged_substeps(self):
         """Substeps of the last dot that used all m* terms without the
         stopping test firing (reads the device counter)."""
-        c = getattr(self, "_last_ctl", None)
-        return 0 if c is None else int(c.view(torch.int32)[10].item())
+        w = self._counters()
+        return 0 if w is None else w[10]
 
     @property
     def terms_executed(self):
         """Taylor terms executed by the last dot (reads the device counter)."""
-        c = getattr(self, "_last_ctl", None)
-        if c is None:
-            return 0
-        return int(c[4].item())
+        w = self._counters()
+        return 0 if w is None else (w[8] & 0xffffffff) | w[9] << 32
 
     def dot(self, v, work_array=None, overwrite_v=False, tol=None):
         """e^{aA} v (html :265-374); numpy in -> numpy out, CUDA tensor in ->
@@ -462,6 +494,8 @@ class ExpmMultiplyParallel:
         self.run_device(F, tol=tol)
         if host:
             res = D.to_host(F)
+            if res.size and np.isnan(res.flat[0]) and self.gave_up:
+                res = D.to_host(self.settle(F, tol))
             res = res.astype(v_dtype, copy=False) if v_dtype.kind == "c" else res.real.astype(v_dtype)
             if overwrite_v:
                 v[...] = res

@@ -114,3 +114,39 @@ def test_small_form_by_entries(cuda, row, one):
     finally:
         ExpmMultiplyParallel.SMALL_MAX_NNZ = old
     assert float((got - ref).norm() / ref.norm()) <= 1e-13
+
+
+@pytest.mark.parametrize("n", [200, 20000])
+def test_small_barrier_gives_up(cuda, monkeypatch, n):
+    """Barriers that may not look even once: the kernel ends by itself, F is NaN
+    as a whole, the counters raise, settle and host results evolve the kept
+    input launch by launch, and the next call is clean."""
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300._lib import QsError
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    rng = np.random.default_rng(n)
+    A = _hermitian(n, True, True, rng)
+    v = rng.normal(size=n) + 1j * rng.normal(size=n)
+    op = ExpmMultiplyParallel(A, a=-0.7j)
+    want = D.to_host(op.dot(D.to_device(v)))
+    assert not op.gave_up
+    terms = op.terms_executed
+    monkeypatch.setattr(ExpmMultiplyParallel, "SMALL_POLLS", 0)
+    F = D.to_device(v).clone()
+    assert op.dot(F, overwrite_v=True) is F and op.gave_up
+    assert bool(torch.isnan(torch.view_as_real(F)).all())
+    for name in ("terms_executed", "nonconverged_substeps"):
+        with pytest.raises(QsError, match="gave up"):
+            getattr(op, name)
+    assert op.settle(F) is F and not op.gave_up
+    assert np.linalg.norm(D.to_host(F) - want) <= 1e-13 * np.linalg.norm(want)
+    assert abs(op.terms_executed - terms) <= op.s
+    host = op.dot(v)                                       # read back: settled by itself
+    assert np.linalg.norm(host - want) <= 1e-13 * np.linalg.norm(want)
+    monkeypatch.setattr(type(op), "partition_source", property(lambda self: "learned"))
+    F = op.run_device(D.to_device(v).clone())              # the learned selection reads its counter
+    assert np.linalg.norm(D.to_host(F) - want) <= 1e-13 * np.linalg.norm(want)
+    monkeypatch.undo()
+    np.testing.assert_array_equal(D.to_host(op.dot(D.to_device(v))), want)
+    assert not op.gave_up and op.terms_executed == terms
