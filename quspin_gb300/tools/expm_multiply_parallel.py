@@ -301,7 +301,7 @@ class ExpmMultiplyParallel:
         tol = float(self._tol if tol is None else tol)
         if one_launch and nvec == 1 and F.is_contiguous() and self._small_operand() is not None \
                 and not torch.cuda.is_current_stream_capturing():
-            return self._run_small(F, tol)
+            return self._run_small(F, tol, work)
         if (work is None and n * nvec <= self.GRAPH_MAX_ELEMS and F.is_contiguous()
                 and not torch.cuda.is_current_stream_capturing()):
             return self._run_graph(F, tol)
@@ -336,10 +336,12 @@ class ExpmMultiplyParallel:
         P, btype = self._operand(1)
         return P if tune_taylor(P, 1, btype) == 0 else None
 
-    def _run_small(self, F, tol):
+    def _run_small(self, F, tol, work=None):
         P = self._small_operand()
         n = self._Ad.shape[0]
-        work, ctl = self._buffers(n, 1, _lib.CPF)
+        wbuf, ctl = self._buffers(n, 1, _lib.CPF)
+        if work is not None:
+            wbuf = work
         sync = self.__dict__.get("_sync")
         if sync is None:
             sync = self._sync = torch.zeros(_lib.load().qs_expm_small_sync_bytes() // 8, dtype=torch.int64,
@@ -354,7 +356,7 @@ class ExpmMultiplyParallel:
         polls = _lib.load().qs_expm_small_polls() if self.SMALL_POLLS is None else self.SMALL_POLLS
         _lib.call("qs_expm_multiply_small_kept", n, P.nnz, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(P.data), P.vcode,
                   D.ptr(F), int(self._s), int(self._m_star), tol, mu.real, mu.imag, D.ptr(consts),
-                  D.ptr(consts[m:m + 1]), D.ptr(work), D.ptr(ctl), D.ptr(sync), D.ptr(self._keep), polls, D.stream())
+                  D.ptr(consts[m:m + 1]), D.ptr(wbuf), D.ptr(ctl), D.ptr(sync), D.ptr(self._keep), polls, D.stream())
         self._last_ctl = ctl
         return F
 

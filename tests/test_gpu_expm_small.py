@@ -150,3 +150,23 @@ def test_small_barrier_gives_up(cuda, monkeypatch, n):
     monkeypatch.undo()
     np.testing.assert_array_equal(D.to_host(op.dot(D.to_device(v))), want)
     assert not op.gave_up and op.terms_executed == terms
+
+
+@pytest.mark.parametrize("n", [300, 30000])
+def test_small_uses_the_callers_work_array(cuda, n):
+    """A device work_array of the result's type holds the term vectors of the
+    one-launch form, as it does those of the other forms."""
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    rng = np.random.default_rng(n)
+    op = ExpmMultiplyParallel(_hermitian(n, False, True, rng), a=-0.7j)
+    assert op._small_operand() is not None
+    v = D.to_device(rng.normal(size=n) + 1j * rng.normal(size=n))
+    want = op.dot(v)
+    for shape in ((2 * n,), (2, n)):
+        work = torch.full(shape, np.pi, dtype=torch.complex128, device="cuda")
+        assert torch.equal(op.dot(v, work_array=work), want)
+        assert not bool((work == np.pi).any())
+    with pytest.raises(ValueError, match="twice"):
+        op.dot(v, work_array=work[0])
