@@ -322,6 +322,7 @@ class ExpmMultiplyParallel:
     # 373, 60 k of 300 1005 / 770; below, 60 k of 40 219 / 289, 1500 of 1500 203 / 218
     SMALL_MAX_ROWS = 65535
     SMALL_MAX_NNZ = 2_400_000
+    SMALL_TABLES = 64       # coefficient tables kept, one per factor and partition
     SMALL_POLLS = None      # looks after which its barriers give up (None: the library's limit, a few seconds)
 
     def _small_operand(self):
@@ -339,19 +340,28 @@ class ExpmMultiplyParallel:
     def _run_small(self, F, tol, work=None):
         P = self._small_operand()
         n = self._Ad.shape[0]
-        wbuf, ctl = self._buffers(n, 1, _lib.CPF)
-        if work is not None:
-            wbuf = work
-        sync = self.__dict__.get("_sync")
-        if sync is None:
-            sync = self._sync = torch.zeros(_lib.load().qs_expm_small_sync_bytes() // 8, dtype=torch.int64,
-                                            device=D.device())
+        # buffers of this form alone, kept as long as the object: other calls
+        # of it, on other streams and of other shapes, never free them
+        ctl, sync = self.__dict__.get("_small_state") or (None, None)
+        if ctl is None:
+            L = _lib.load()
+            ctl = torch.zeros(max(L.qs_expm_ctl_bytes() // 8, 1) + 1, dtype=torch.int64, device=D.device())
+            sync = torch.zeros(L.qs_expm_small_sync_bytes() // 8, dtype=torch.int64, device=D.device())
             self._keep = torch.empty(n, dtype=torch.complex128, device=D.device())
+            self._small_state = ctl, sync
+        wbuf = work
+        if wbuf is None:
+            wbuf = self.__dict__.get("_small_work")
+            if wbuf is None:
+                wbuf = self._small_work = torch.empty(2 * n, dtype=torch.complex128, device=D.device())
         key = (complex(self._a), complex(self._mu), int(self._s), int(self._m_star))
-        kept = self.__dict__.get("_small_consts")
-        if kept is None or kept[0] != key:
-            kept = self._small_consts = (key, self._const_table())
-        consts, m = kept[1], max(int(self._m_star), 1)
+        tables = self.__dict__.setdefault("_small_consts", {})
+        if key not in tables:
+            if len(tables) >= self.SMALL_TABLES:
+                torch.cuda.synchronize()        # launches on any stream may still read them
+                tables.clear()
+            tables[key] = self._const_table()
+        consts, m = tables[key], max(int(self._m_star), 1)
         mu = complex(self._mu)
         polls = _lib.load().qs_expm_small_polls() if self.SMALL_POLLS is None else self.SMALL_POLLS
         _lib.call("qs_expm_multiply_small_kept", n, P.nnz, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(P.data), P.vcode,

@@ -170,3 +170,29 @@ def test_small_uses_the_callers_work_array(cuda, n):
         assert not bool((work == np.pi).any())
     with pytest.raises(ValueError, match="twice"):
         op.dot(v, work_array=work[0])
+
+
+def test_small_buffers_outlive_other_calls(cuda):
+    """What a launch of the one-launch form reads and writes is not freed by
+    later calls of the same object, which another stream may issue while it
+    runs: a call with several vectors, or with another factor."""
+    from quspin_gb300 import _device as D
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    rng = np.random.default_rng(3)
+    n = 50000
+    op = ExpmMultiplyParallel(_hermitian(n, False, True, rng), a=-0.5j)
+    op.GRAPH_MAX_ELEMS = 0
+    v = D.to_device(rng.normal(size=n) + 1j * rng.normal(size=n))
+    want = op.dot(v)
+    held = [t.data_ptr() for t in (*op._small_state, op._keep, op._small_work, *op._small_consts.values())]
+    op.dot(v.reshape(n, 1).expand(n, 3).contiguous())
+    op.set_a(-0.25j)
+    op.dot(v)
+    op.set_a(-0.5j)
+    assert bool((op.dot(v) == want).all())
+    now = [t.data_ptr() for t in (*op._small_state, op._keep, op._small_work, *op._small_consts.values())]
+    assert now[:len(held)] == held
+    for i in range(op.SMALL_TABLES + 3):
+        op.set_a(-0.01j * (i + 1))
+        op.dot(v)
+    assert len(op._small_consts) <= op.SMALL_TABLES
