@@ -102,6 +102,9 @@ def _recurrence(op, q0, m, eps, Q=None, reorth=False):
     Q: optional device [m, n] tensor receiving the Lanczos vectors.  Returns
     (a, b, m_eff) with a, b host arrays."""
     n = q0.shape[0]
+    shape = tuple(getattr(op.A, "shape", (n, n)))
+    if shape != (n, n):      # the kernels take the operator's size for the vectors'
+        raise ValueError("matrix dimension mismatch with shapes: {0} and {1}.".format((n,), shape))
     cplx = int(q0.dtype == torch.complex128)
     n2 = n * (2 if cplx else 1)
     L = _lib.load()

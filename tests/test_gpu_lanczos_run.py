@@ -66,3 +66,23 @@ def test_run_stops_in_invariant_subspace(cuda, reorth):
     assert Q.shape[0] in (6, 5)                        # b vanishes after the sixth vector
     k = Q.shape[0]
     np.testing.assert_allclose(np.sort(E), np.linalg.eigvalsh(A.toarray()[:k, :k]), rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("form", ["hamiltonian", "csr", "linop", "mixed"])
+@pytest.mark.parametrize("off", [-3, 4])
+def test_start_vector_of_another_size_is_refused(cuda, form, off):
+    """The run and the steps take the operator's row count for the vectors'
+    length, so a start vector of another length is an error before any launch."""
+    from quspin_gb300 import hamiltonian, quantum_LinearOperator, spin_basis_general
+    from quspin_gb300.tools import lanczos_full, lanczos_iter
+    from tests.models import xxz_static
+    b = spin_basis_general(10, Nup=5, pauli=0)
+    H = hamiltonian(xxz_static(10), [], basis=b, dtype=np.float64)
+    A = {"hamiltonian": H, "csr": H.static, "mixed": H,
+         "linop": quantum_LinearOperator(xxz_static(10), basis=b, dtype=np.float64)}[form]
+    v = np.ones(b.Ns + off)
+    for reorth in (False, True):
+        with pytest.raises(ValueError, match="mismatch"):
+            lanczos_full(A, v, 6, reorth=reorth, precision="mixed" if form == "mixed" else "double")
+    with pytest.raises(ValueError, match="mismatch"):
+        lanczos_iter(A, v, 6)
