@@ -29,19 +29,25 @@ static int lz_blocks(int64_t n)
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-// x / b with b's reciprocal at hand: one correction step on the exact
-// remainder, three FP64 instructions where a division takes about ten.  `fast`
-// says that b and its reciprocal are well inside the normal range.
-__device__ __forceinline__ double div_by(double x, double b, double inv, bool fast)
-{
-    if (!fast) return x / b;
-    const double q = x * inv;
-    return fma(fma(-q, b, x), inv, q);
-}
+// x / b, correctly rounded, with b's correctly rounded reciprocal at hand: a
+// product and one correction by the remainder (N. Brisebarre, J.-M. Muller and
+// S. K. Raina, "Accelerating correctly rounded floating-point division when the
+// divisor is known in advance", IEEE Trans. Comput. 53 (2004) 1069-1072, after P.
+// Markstein, IBM J. Res. Dev. 34 (1990) 111-119), three FP64 instructions where a
+// division takes about ten.  It holds while nothing leaves the normal range: with
+// x and b between 2^-500 and 2^501 in size the quotient stays between 2^-1001 and
+// 2^1001 and the remainder is a multiple of 2^-606.  Zeros are quotients of their
+// own; all else (x or b beyond that, infinities, NaN) is divided.
 __device__ __forceinline__ bool div_fast(double b)
 {
-    const int e = (__double2hiint(b) >> 20) & 0x7ff;
-    return e > 123 && e < 1923;
+    return (unsigned)(((__double2hiint(b) >> 20) & 0x7ff) - 523) <= 1000u;
+}
+__device__ __forceinline__ double div_by(double x, double b, double inv, bool fast)
+{
+    const double q = x * inv;
+    if (fast && div_fast(x)) return fma(fma(-q, b, x), inv, q);
+    if (fast && x == 0.0) return q;
+    return x / b;
 }
 
 // q = r / b[i-1] (also the first step with b = norm of v0 when i == 0)
