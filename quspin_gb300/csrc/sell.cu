@@ -244,7 +244,10 @@ __global__ void __launch_bounds__(ST, SOCC) sell_lz_kernel(LzProduct p, const in
 // instructions run only where the FP32 value says that some lane may pass what
 // the warp has seen (an FP32 square is within a few 2^-23 of the FP64 one, the
 // margin 2^-18): the maximum is the same to the bit, at about log of the number
-// of slices instead of every slice.  NaN counts as nothing, as in fmax.
+// of slices instead of every slice.  Squares below the normal float range have
+// no such bound and count as nothing seen, so that what follows passes; against
+// a larger one, whose margin is 2^-144 or more, they cannot win.  NaN counts as
+// nothing, as in fmax.
 struct MaxSquare {
     double best = 0.0;
     uint32_t seen = 0u;      // bits of the largest FP32 value of the warp, less the margin
@@ -253,7 +256,9 @@ struct MaxSquare {
         const float q = __fmaf_rn(a, a, __fmul_rn(b, b));
         const uint32_t top = __reduce_max_sync(0xffffffffu, q == q ? __float_as_uint(q) : 0u);
         if (top < seen) return false;
-        seen = top >= 0x7f800000u ? top : __float_as_uint(__fmul_rn(__uint_as_float(top), 1.0f - 0x1p-18f));
+        seen = top < 0x00800000u    ? 0u
+               : top >= 0x7f800000u ? top
+                                    : __float_as_uint(__fmul_rn(__uint_as_float(top), 1.0f - 0x1p-18f));
         return true;
     }
     __device__ __forceinline__ void take(double a, double b) { best = fmax(best, __dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b))); }

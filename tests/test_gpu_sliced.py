@@ -177,3 +177,35 @@ def test_tuned_pick(cuda, kind):
     ref._pick = ref.A_device.paired()
     ref._pick.__dict__.setdefault("_tuned", {})[("taylor", 1, _lib.CPF)] = encode(4, 1)
     assert np.linalg.norm(out - D.to_host(ref.dot(D.to_device(v)))) <= 1e-13 * np.linalg.norm(out)
+
+
+@pytest.mark.parametrize("power", [0, -40, -62, -63, -64, -70, -74, -100])
+def test_term_norm_is_the_largest_modulus(cuda, power):
+    """The stopping test's norm of a term, bit for bit, however small the term
+    is next to its scale: the first half of the rows hold the modulus whose FP32
+    square is the larger near 2^-140, the second half the larger one."""
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300 import _lib
+    from quspin_gb300.sparse import SLICED, SlicedCSR
+    from quspin_gb300.tune import encode
+    n = 640000                                              # several slices to every warp
+    M, P = _packed(sp.identity(n, format="csr"))
+    limit, SlicedCSR.MAX_PADDING = SlicedCSR.MAX_PADDING, 40.0
+    try:
+        S = P.sliced()
+    finally:
+        SlicedCSR.MAX_PADDING = limit
+    small, large = np.float32([1.0064243, 1.0005476]), np.float32([1.0052148, 1.0023396])
+    b = np.zeros((n, 4), np.float32)
+    b[:n // 2, 0::2], b[n // 2:, 0::2] = small, large
+    b0 = D.to_device(b)
+    b1, F = torch.empty_like(b0), torch.ones(n, dtype=torch.complex128, device="cuda")
+    ctl = torch.zeros(_lib.load().qs_expm_ctl_bytes() // 8 + 1, dtype=torch.int64, device="cuda")
+    c = torch.tensor([2.0**power + 0j], dtype=torch.complex128, device="cuda")
+    _lib.call("qs_taylor_term", n, S.nnz, D.ptr(S.indptr), 0, D.ptr(S.indices), D.ptr(S.data), S.vcode, D.ptr(b0),
+              D.ptr(b1), _lib.CPF, D.ptr(F), 1, 0.0, 0.0, D.ptr(c), 0, 0.0, D.ptr(ctl), encode(2, 2) | SLICED,
+              D.stream())
+    np.testing.assert_array_equal(D.to_host(b1), b * np.float32(2.0**power))
+    h = large.astype(np.float64)
+    assert ctl[:1].view(torch.float64).item() == np.sqrt(h[0] * h[0] + h[1] * h[1]) * 2.0**power
