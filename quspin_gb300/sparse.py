@@ -399,12 +399,17 @@ class PairedCSR:
 
     def packed(self):
         """The PackedCodedCSR form of this coded operand (cached), or None
-        when it does not apply (plain values, int64 indices, >= 2^23 columns)."""
+        when it does not apply (plain values, int64 indices, >= 2^23 columns)
+        or there is no memory for its words; every product runs on this form
+        as well."""
         if not self.coded or self.idx64 or self.shape[1] >= PackedCodedCSR.MAX_COLS:
             return None
         p = self.__dict__.get("_packed")
         if p is None:
-            p = PackedCodedCSR(self)
+            try:
+                p = PackedCodedCSR(self)
+            except torch.OutOfMemoryError:
+                return None
             self._packed = p
         return p
 
@@ -469,10 +474,21 @@ class PackedCodedCSR:
     def sliced(self):
         """The SlicedCSR form of this operand (cached), or None when it does
         not apply (a row of more than 128 nonzeros, or rows so uneven that
-        the slices would hold half as much again)."""
+        the slices would hold half as much again) or there is no memory for
+        its words."""
         if "_sliced" not in self.__dict__:
             self._sliced = SlicedCSR.build(self)
         return self._sliced
+
+    def keep_sliced(self, user):
+        """Records that ``user`` (None: nobody) has chosen the sliced form after
+        timing it; gives its words, as large as this operand's, back when nobody
+        has.  ``sliced`` builds them again where they are asked for."""
+        users = self.__dict__.setdefault("_sliced_users", set())
+        if user is not None:
+            users.add(user)
+        if not users and self.__dict__.get("_sliced") is not None:
+            del self._sliced
 
     @property
     def nnz(self):
@@ -504,21 +520,21 @@ class SlicedCSR:
         if n == 0 or nnz == 0:
             return None
         slices = (n + 31) // 32
-        sptr = torch.zeros(slices + 1, dtype=torch.int64, device=D.device())
-        most = torch.zeros(1, dtype=torch.int32, device=D.device())
-        _lib.call("qs_sell_count", n, D.ptr(P.indptr), D.ptr(sptr[1:]), D.ptr(most), D.stream())
-        scr = torch.empty(max(_lib.load().qs_scan_scratch_elems(slices), 1), dtype=torch.int64, device=D.device())
-        _lib.call("qs_scan_inclusive_i64", D.ptr(sptr[1:]), slices, D.ptr(scr), D.stream())
-        groups = int(sptr[-1].item())
-        if int(most.item()) > cls.MAX_ROW or groups * 128 > cls.MAX_PADDING * nnz + 4096:
-            return None
-        S = cls()
-        S.indptr, S.data, S.shape, S.idx64 = sptr, P.data, P.shape, 0
-        S._nnz, S.complex, S.dtype, S.distinct, S.coded = nnz, P.complex, P.dtype, P.distinct, True
         try:
-            S.indices = torch.empty(groups * 128, dtype=torch.int32, device=D.device())
+            sptr = torch.zeros(slices + 1, dtype=torch.int64, device=D.device())
+            most = torch.zeros(1, dtype=torch.int32, device=D.device())
+            _lib.call("qs_sell_count", n, D.ptr(P.indptr), D.ptr(sptr[1:]), D.ptr(most), D.stream())
+            scr = torch.empty(max(_lib.load().qs_scan_scratch_elems(slices), 1), dtype=torch.int64, device=D.device())
+            _lib.call("qs_scan_inclusive_i64", D.ptr(sptr[1:]), slices, D.ptr(scr), D.stream())
+            groups = int(sptr[-1].item())
+            if int(most.item()) > cls.MAX_ROW or groups * 128 > cls.MAX_PADDING * nnz + 4096:
+                return None
+            words = torch.empty(groups * 128, dtype=torch.int32, device=D.device())
         except torch.OutOfMemoryError:      # the packed form serves as well
             return None
+        S = cls()
+        S.indptr, S.indices, S.data, S.shape, S.idx64 = sptr, words, P.data, P.shape, 0
+        S._nnz, S.complex, S.dtype, S.distinct, S.coded = nnz, P.complex, P.dtype, P.distinct, True
         _lib.call("qs_sell_fill", n, D.ptr(P.indptr), D.ptr(P.indices), D.ptr(sptr), groups, D.ptr(S.indices),
                   D.stream())
         return S

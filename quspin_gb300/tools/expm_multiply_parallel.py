@@ -232,13 +232,19 @@ class ExpmMultiplyParallel:
             Pk = P.packed() if P.shape[0] >= 65536 else None
             if Pk is not None:
                 from ..tune import tune_taylor
-                S = Pk.sliced()
+                # what an earlier evolution of this matrix found stays: the
+                # losing sliced words are not built again
+                S = Pk.sliced() if Pk.__dict__.get("_term_form") != "packed" else None
+                known = "_term_form" in Pk.__dict__
                 key, best = ("taylor", 1, _lib.CPF), None
-                for form in (P, Pk) if S is None else (Pk, S):
+                for form in ((S or Pk,) if known else (P, Pk) if S is None else (Pk, S)):
                     tune_taylor(form, 1, _lib.CPF)
                     t = form.__dict__.get("_tuned_ms", {}).get(key)
                     if t is not None and (best is None or t < best):
                         pick, best = form, t
+                if S is not None:
+                    Pk._term_form = "sliced" if pick is S else "packed"
+                    Pk.keep_sliced("term" if pick is S else None)
             self._pick = pick
         return pick, _lib.CPF
 

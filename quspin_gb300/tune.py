@@ -6,7 +6,8 @@ distribution and on how the gathers of the vector spread over L2, so it is
 measured: a handful of candidate shapes around the nnz/row heuristic are timed
 with CUDA events on the actual matrix and the fastest is kept on the matrix
 object.  For one vector on a packed operand its sliced form (csrc/sell.cu, one
-shape, launch code bit ``SLICED``) is timed with them.  Matrices smaller than ``MIN_ROWS`` keep the heuristic shape.
+shape, launch code bit ``SLICED``) is timed with them, and kept only where it
+wins.  Matrices smaller than ``MIN_ROWS`` keep the heuristic shape.
 """
 from __future__ import annotations
 
@@ -112,7 +113,8 @@ def tune_spmv(M, nvec=1, xdtype=np.complex128, precision="double", operand=None)
     if (nvec == 1 and np.dtype(xdtype).kind == "c" and getattr(operand, "padded", False)
             and getattr(operand, "vcode", None) in (_lib.PF8P, _lib.CPF8P)):
         codes += [encode(G, 1) | (6 << 20) for G in (2, 4)]      # column words read four per load
-    if nvec == 1 and _sliced(operand) is not None:
+    sliced = nvec == 1 and _sliced(operand) is not None
+    if sliced:
         # against the row hand-out shapes that win where rows share few lines
         codes = [c for c in codes if c >> 20] or [encode(G, U) for G in (2, 4) for U in (1, 2)]
         codes.append(encode(2, 1) | SLICED)
@@ -120,6 +122,8 @@ def tune_spmv(M, nvec=1, xdtype=np.complex128, precision="double", operand=None)
         t = _time(lambda: M.matvec_into(x, y, group=code, precision=precision, operand=operand))
         if best_t is None or t < best_t:
             best, best_t = code, t
+    if sliced:
+        operand.keep_sliced("product" if best & SLICED else None)
     cache[key] = best
     return best
 

@@ -209,3 +209,86 @@ def test_term_norm_is_the_largest_modulus(cuda, power):
     np.testing.assert_array_equal(D.to_host(b1), b * np.float32(2.0**power))
     h = large.astype(np.float64)
     assert ctl[:1].view(torch.float64).item() == np.sqrt(h[0] * h[0] + h[1] * h[1]) * 2.0**power
+
+
+@pytest.mark.parametrize("wins", [False, True])
+def test_sliced_words_kept_only_where_they_win(cuda, monkeypatch, wins):
+    """The words are as large as the packed operand: the tuner, which builds
+    them to time them, keeps them for the products and the terms that run on
+    them and gives them back otherwise; a second evolution does not build them
+    again to find the same."""
+    from quspin_gb300 import _device as D
+    from quspin_gb300 import tune
+    from quspin_gb300.sparse import SLICED, DeviceCSR, SlicedCSR
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    built, build = [], SlicedCSR.build.__func__
+    monkeypatch.setattr(SlicedCSR, "build", classmethod(lambda cls, P: built.append(1) or build(cls, P)))
+    clock = [1e3]
+
+    def time(fn, reps=5):                                   # the sliced form is timed last
+        fn()
+        clock[0] *= 0.99 if wins else 1.01
+        return clock[0]
+    monkeypatch.setattr(tune, "_time", time)
+    rng = np.random.default_rng(5)
+    n = 65600
+    A = _matrix(n, False, "even", rng)
+    x = rng.normal(size=n) + 1j * rng.normal(size=n)
+    M = DeviceCSR.from_scipy(A)
+    P = M.paired().packed()
+    y = M.dot(D.to_device(x))                               # small: no float pairs, no tuning
+    M.matvec_into(D.to_device(x), y, precision="double")
+    assert bool(M._tuned[("spmv", 1, np.dtype(np.complex128).str, "double", P.vcode)] & SLICED) == wins
+    assert ("_sliced" in P.__dict__) == wins and len(built) == 1
+    assert np.all(abs(D.to_host(y) - A @ x) <= 1e-13 * (abs(A) @ abs(x)))
+    M = DeviceCSR.from_scipy(A)
+    P = M.paired().packed()
+    built.clear()
+    for _ in range(2):
+        op = ExpmMultiplyParallel(M, a=-0.1j)
+        op.set_partition(6, 1)
+        assert (op._operand(1)[0] is P.__dict__.get("_sliced")) == wins
+    assert ("_sliced" in P.__dict__) == wins and len(built) == 1
+
+
+@pytest.mark.parametrize("what", ["packed", "sliced", "pointers"])
+def test_forms_without_memory(cuda, monkeypatch, what):
+    """No memory for the packed words, the sliced words or the slice pointers:
+    the operand of before serves, for one vector and several."""
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300 import sparse
+    from quspin_gb300.sparse import DeviceCSR
+    from quspin_gb300.tools import ExpmMultiplyParallel
+    rng = np.random.default_rng(6)
+    n = 65600
+    A = _matrix(n, False, "even", rng)
+    M = DeviceCSR.from_scipy(A)
+    P = M.paired()
+    V = rng.normal(size=(n, 3)) + 1j * rng.normal(size=(n, 3))
+    op = ExpmMultiplyParallel(DeviceCSR.from_scipy(A), a=-0.1j)
+    op.set_partition(6, 1)
+    want = [D.to_host(op.dot(D.to_device(v))) for v in (V[:, 0].copy(), V)]
+
+    class Full:                                             # the allocations of the class under test fail
+        OutOfMemoryError = torch.OutOfMemoryError
+        def __getattr__(self, name):
+            if name == {"packed": "zeros", "sliced": "empty", "pointers": "zeros"}[what]:
+                return self.fail
+            return getattr(torch, name)
+        @staticmethod
+        def fail(*a, dtype=None, **k):
+            if dtype is {"packed": torch.int32, "sliced": torch.int32, "pointers": torch.int64}[what] and a[0] > 1:
+                raise torch.OutOfMemoryError("no memory")
+            return getattr(torch, {"packed": "zeros", "sliced": "empty", "pointers": "zeros"}[what])(*a, dtype=dtype, **k)
+    op = ExpmMultiplyParallel(M, a=-0.1j)
+    op.set_partition(6, 1)
+    monkeypatch.setattr(sparse, "torch", Full())
+    got = [D.to_host(op.dot(D.to_device(v))) for v in (V[:, 0].copy(), V)]
+    assert (P.packed() is None) == (what == "packed")
+    assert what == "packed" or P.packed().sliced() is None
+    for g, w in zip(got, want):
+        assert np.linalg.norm(g - w) <= 1e-13 * np.linalg.norm(w)
+    y = torch.empty(n, dtype=torch.complex128, device="cuda")
+    M.matvec_into(D.to_device(V[:, 0].copy()), y, precision="double")
+    assert np.all(abs(D.to_host(y) - A @ V[:, 0]) <= 1e-13 * (abs(A) @ abs(V[:, 0])))
