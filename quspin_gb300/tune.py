@@ -20,6 +20,16 @@ from .sparse import SLICED
 
 MIN_ROWS = 65536
 
+# From these row counts on, the sliced form of a packed operand is timed against
+# a few row hand-out shapes instead of all of them (0.28 s at 159 M nonzeros).
+# Measured on even rows of 8 to 100 nonzeros with random, banded, shifted and
+# bit-flip columns, real and complex: the term's sliced form is the fastest of
+# all at 0.5 M rows and more (6 to 60% ahead), while below some 0.2 M another
+# shape wins by up to 10% (70 k rows of 8: 14.9 against 16.5 us); the product's
+# from 0.13 M on is within 1% of the best.  The coded operand (a code byte beside
+# each index) is never ahead of both by more than 1% and is not timed.
+FEW_ROWS_TERM, FEW_ROWS_PRODUCT = 1 << 18, 1 << 17
+
 
 def encode(G, U):
     return int(G) | (int(U) << 8)
@@ -115,8 +125,8 @@ def tune_spmv(M, nvec=1, xdtype=np.complex128, precision="double", operand=None)
         codes += [encode(G, 1) | (6 << 20) for G in (2, 4)]      # column words read four per load
     sliced = nvec == 1 and _sliced(operand) is not None
     if sliced:
-        # against the row hand-out shapes that win where rows share few lines
-        codes = [c for c in codes if c >> 20] or [encode(G, U) for G in (2, 4) for U in (1, 2)]
+        if n >= FEW_ROWS_PRODUCT:
+            codes = [c for c in codes if c >> 20] or [encode(G, U) for G in (2, 4) for U in (1, 2)]
         codes.append(encode(2, 1) | SLICED)
     for code in codes:
         t = _time(lambda: M.matvec_into(x, y, group=code, precision=precision, operand=operand))
@@ -160,9 +170,7 @@ def tune_taylor(M, nvec, btype):
     if getattr(M, "vcode", None) in (_lib.PF8S, _lib.CPF8S):
         cands = [(2, 2, SLICED >> 16)]
     rows = r32_candidates(M, nvec, btype)
-    if nvec == 1 and _sliced(M) is not None:
-        # the form to beat is the sliced one: time the shapes that win where
-        # rows share few lines (all of them cost 0.28 s at 159 M nonzeros)
+    if nvec == 1 and n >= FEW_ROWS_TERM and _sliced(M) is not None:
         rows = [c for c in rows if c in ((4, 1), (6, 1), (6, 2))]
     cands += [({1: 4, 2: 2, 3: 8, 4: 2, 5: 4, 6: 2, 7: 4}[shape], 2, (shape << 4) | (occ << 2))
               for shape, occ in rows]

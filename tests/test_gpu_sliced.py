@@ -292,3 +292,32 @@ def test_forms_without_memory(cuda, monkeypatch, what):
     y = torch.empty(n, dtype=torch.complex128, device="cuda")
     M.matvec_into(D.to_device(V[:, 0].copy()), y, precision="double")
     assert np.all(abs(D.to_host(y) - A @ V[:, 0]) <= 1e-13 * (abs(A) @ abs(V[:, 0])))
+
+
+def test_tuner_times_every_shape_of_smaller_operands(cuda, monkeypatch):
+    """Below the row counts from which the sliced form always leads, it is
+    timed against all row hand-out shapes of the packed operand; from there on
+    against a few of them."""
+    from quspin_gb300 import _lib, tune
+    from quspin_gb300.sparse import DeviceCSR
+    n = 65600
+    A = _matrix(n, False, "even", np.random.default_rng(7))
+    timed = []
+    monkeypatch.setattr(tune, "_time", lambda fn, reps=5: timed.append(1) or 1.0)
+    count = {}
+    for few in (False, True):
+        monkeypatch.setattr(tune, "FEW_ROWS_PRODUCT", n + (not few))
+        monkeypatch.setattr(tune, "FEW_ROWS_TERM", n + (not few))
+        M = DeviceCSR.from_scipy(A)
+        P = M.paired().packed()
+        for xdtype in (np.complex128, np.float64):
+            timed.clear()
+            tune.tune_spmv(M, 1, xdtype, "double", operand=P)
+            count[few, xdtype] = len(timed)
+        timed.clear()
+        tune.tune_taylor(P, 1, _lib.CPF)
+        count[few, "term"] = len(timed)
+    full = len(tune._candidates(n, A.nnz, 1))
+    assert count[False, np.complex128] == full + 3 and count[False, np.float64] == full + 1
+    assert count[True, np.complex128] == 3 and count[True, np.float64] == 5
+    assert count[False, "term"] == len(tune.r32_candidates(P, 1, _lib.CPF)) and count[True, "term"] == 3
