@@ -259,8 +259,9 @@ int vl_idx(const LpTerm &a)
 // 10% slower, and more at five, 15%).
 int vl_taylor_term(const LpTerm &a, bool multi)
 {
-    if (a.nvec < 2 || a.nvec >= (1 << 27) || a.staged < 1 || a.staged > 3) return QS_ERR_ARG;
+    if (a.nvec < 2 || a.staged < 1 || a.staged > 3) return QS_ERR_ARG;
     if (multi && a.idx64) return QS_ERR_ARG;
+    if (a.nvec >= (1 << 27)) return lp_taylor_term(a, multi);       // strides beyond 32 bits: the row hand-out
     if (a.btype == QS_CPF) {
         switch (a.dtype) {
         case QS_PF: return multi ? vl_idx<ModePF, pf, true>(a) : vl_idx<ModePF, pf, false>(a);

@@ -375,7 +375,7 @@ int spmm_go(const SpmvArgs &a)
     const int64_t rows = 8 * (32 / (VL * split));       // per block and sweep
     // with few rows the sweeps go to blocks of their own, too
     int64_t apart = lanes / (a.n * VL * split);
-    if (apart > 64) apart = 64;
+    if (apart > 65535) apart = 65535;
     if (apart > (a.nvec + VL - 1) / VL) apart = (a.nvec + VL - 1) / VL;
     const dim3 grid(qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident), (unsigned)(apart < 1 ? 1 : apart));
     k<<<grid, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, a.x, (YT *)a.y, a.nvec, VL,
@@ -398,6 +398,9 @@ int spmv_nb(const SpmvArgs &a)
             }
             return spmv_go<M, DV, XC, YT, IT, 1, VM>(a);
         }
+        // a row of the vectors beyond 4 GB
+        if (a.nvec > (int64_t)(0xffffffffu / (XC ? sizeof(typename M::BE) : sizeof(typename M::S))))
+            return spmm_go<M, DV, XC, YT, IT, VM, 1, uint64_t>(a);
         if (a.nvec <= 3) return spmm_go<M, DV, XC, YT, IT, VM, 2>(a);
         return spmm_go<M, DV, XC, YT, IT, VM, 1>(a);
     }
@@ -489,7 +492,7 @@ extern "C" int qs_csr_matvec_pairs(int64_t n, int64_t nnz, const void *indptr, i
                                    double a_re, double a_im, int overwrite, int group, void *xs, void *norm,
                                    void *stream)
 {
-    if (n < 0 || nvec < 1 || nvec >= (1 << 27) || (n > 0 && (!indptr || !x || !y || !xs || !norm))) return QS_ERR_ARG;
+    if (n < 0 || nvec < 1 || (n > 0 && (!indptr || !x || !y || !xs || !norm))) return QS_ERR_ARG;
     if (n == 0) return QS_OK;
     const bool xc = xtype == QS_C128;
     if (!xc && xtype != QS_F64) return QS_ERR_ARG;

@@ -75,8 +75,8 @@ def lanes_operand(M, nvec, code):
     """The operand a launch code reads: with the vectors across the lanes
     (several vectors, shape bits set or code 0) a coded operand's packed form
     where it has one -- a word per nonzero instead of an index and a code
-    byte; otherwise M itself."""
-    if nvec == 1 or not getattr(M, "coded", False) or (code and not (code >> 20) & 7):
+    byte; otherwise M itself, as for vectors too many for that kernel."""
+    if nvec == 1 or nvec >= 1 << 27 or not getattr(M, "coded", False) or (code and not (code >> 20) & 7):
         return M
     pack = getattr(M, "packed", None)
     P = pack() if pack is not None else None
