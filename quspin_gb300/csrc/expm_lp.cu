@@ -447,7 +447,8 @@ __global__ void __launch_bounds__(256) taylor_norm1_kernel(int64_t n, cdbl *__re
         const int E = (int)(__reduce_max_sync(0xffffffffu, hx > hy ? hx : hy) >> 20);
         bool exact = E == 0 || E == 0x7ff;         // zeros and subnormals; infinities and NaN
         if (!exact) {
-            const unsigned long long seen = *((volatile unsigned long long *)&s_seen);
+            // one lane's look for the warp: others may raise the word meanwhile
+            const unsigned long long seen = __shfl_sync(0xffffffffu, *((volatile unsigned long long *)&s_seen), 0);
             const int Ks = (int)(seen >> 32), K = E > Ks ? E : Ks;
             const float a = d2f_scaled(f.x, K - 1023), b = d2f_scaled(f.y, K - 1023);
             const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(__fmaf_rn(a, a, __fmul_rn(b, b))));
