@@ -1384,10 +1384,16 @@ __global__ void csr_compact_kernel(int64_t Ns, const int64_t *__restrict__ rowpt
 
 // Term slices and blocks of the element kernels: slices of at least eight
 // terms until every resident warp (16 blocks of 4 warps per SM) has a task.
+// A sector so small that this leaves three quarters of the chip idle takes
+// smaller ones, down to a term: a slice's searches run one after another, and
+// with a group of 128 elements by the odometer one takes some 20 us (matrix-free
+// apply of the 4 x 4 lattice with five maps, 199 kets: 0.27 ms in slices of eight
+// terms, 0.15 so; 4 x 5, 1392 kets: 0.30 and 0.21).
 static int elem_slices(int64_t Ns, int T)
 {
     const int64_t groups = (Ns + 31) / 32, want = (int64_t)qs_num_sms() * 16 * ELEM_WARPS;
     int64_t s = (want + groups - 1) / groups, most = (T + 7) / 8;
+    if (most * groups < want / 4) most = want / 4 / groups < T ? want / 4 / groups : T;
     return (int)(s < 1 ? 1 : (s > most ? (most < 1 ? 1 : most) : s));
 }
 struct ElemLaunch {
