@@ -89,6 +89,15 @@ static inline int vl_split(int64_t n, int64_t nnz, int VL, int64_t lanes = 10000
 
 constexpr int VB = 4;      // nonzeros of a row in flight
 
+// Chains of a row's sum in one lane, places taken in turn, as the lanes of a row
+// hand-out are chains of their own.  Float pairs take two (four spill: a product of
+// 8 vectors 45.3 -> 47.6 us); plain floats four, summed every VFLUSH batches, since
+// their roundings are what a result is made of: RMS error of a complex64 product
+// of 8 vectors, rows of 24 and 400, 9.3e-8 and 3.6e-7 with two chains, 6.9e-8 and
+// 9.4e-8 so (row hand-out: 6.6e-8 to 9.3e-8 by its lanes, and 1.1e-7).
+template <class M> constexpr int VCHAINS = std::is_same<M, ModeF32>::value ? 4 : 2;
+constexpr int VFLUSH = 4;
+
 // A lane's place in its warp: vector v of part `part` of row `grp` of `rows`;
 // lane0: the first lane of its VL.
 struct VlPlace {
@@ -111,9 +120,10 @@ template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool FULL, c
 __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, const DV *__restrict__ data,
                                          const uint8_t *__restrict__ codes, const DV *tab,
                                          const char *__restrict__ x, ST stride, IT k, int left,
-                                         typename M::S (&ar)[2], typename M::S (&ai)[2])
+                                         typename M::S (&ar)[VCHAINS<M>], typename M::S (&ai)[VCHAINS<M>])
 {
     using XE = typename std::conditional<XC, typename M::BE, typename M::S>::type;
+    constexpr int NC = VCHAINS<M>;
     XE xe[VB];
     DV d[VB];
 #pragma unroll
@@ -129,8 +139,8 @@ __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, 
 #pragma unroll
     for (int u = 0; u < VB; u++) {
         if (FULL || u < left) {
-            if constexpr (XC) vmul_acc<M>(ar[u & 1], ai[u & 1], d[u], xe[u]);
-            else rmul_acc<M>(ar[u & 1], ai[u & 1], d[u], xe[u]);
+            if constexpr (XC) vmul_acc<M>(ar[u % NC], ai[u % NC], d[u], xe[u]);
+            else rmul_acc<M>(ar[u % NC], ai[u % NC], d[u], xe[u]);
         }
     }
 }
@@ -172,11 +182,12 @@ __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, 
             word[i] = loads && k < len ? (uint32_t)__ldcs(indices + k0 + k) : 0u;
         }
     };
-    // even and odd places apart, as two lanes of a row hand-out: half the
-    // roundings that one chain collects
-    typename M::S ar[2] = {M::zero(), M::zero()}, ai[2] = {M::zero(), M::zero()};
+    typename M::S ar[VCHAINS<M>], ai[VCHAINS<M>];
+#pragma unroll
+    for (int i = 0; i < VCHAINS<M>; i++) ar[i] = ai[i] = M::zero();
     fetch(0);
-    for (int b = 0; b < most; b += step) {
+    typename M::S tr = M::zero(), ti = M::zero();
+    for (int b = 0, t = 1; b < most; b += step, t++) {
         uint32_t cur[WPL];
 #pragma unroll
         for (int i = 0; i < WPL; i++) cur[i] = word[i];
@@ -185,9 +196,24 @@ __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, 
             vl_batch<M, DV, XC, IT, VMODE, WPL, true>(cur, lane0, data, codes, tab, xb, stride, k0 + b, VB, ar, ai);
         else
             vl_batch<M, DV, XC, IT, VMODE, WPL, false>(cur, lane0, data, codes, tab, xb, stride, k0 + b, len - b, ar, ai);
+        if constexpr (VCHAINS<M> == 4) {
+            if (t % VFLUSH == 0) {
+                tr = M::add(tr, M::add(M::add(ar[0], ar[2]), M::add(ar[1], ar[3])));
+                ti = M::add(ti, M::add(M::add(ai[0], ai[2]), M::add(ai[1], ai[3])));
+#pragma unroll
+                for (int i = 0; i < VCHAINS<M>; i++) ar[i] = ai[i] = M::zero();
+            }
+        }
     }
-    sr = M::merge(ar[0], ar[1]);
-    si = M::merge(ai[0], ai[1]);
+#pragma unroll
+    for (int h = VCHAINS<M> / 2; h > 0; h /= 2)
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            ar[i] = M::merge(ar[i], ar[i + h]);
+            ai[i] = M::merge(ai[i], ai[i + h]);
+        }
+    sr = VCHAINS<M> == 4 ? M::add(tr, ar[0]) : ar[0];
+    si = VCHAINS<M> == 4 ? M::add(ti, ai[0]) : ai[0];
     for (int o = 1; o < split; o <<= 1) {
         const int from = (threadIdx.x & 31) + o * VL;
         sr = M::merge(sr, M::shfl(sr, from));

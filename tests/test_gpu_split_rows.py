@@ -69,3 +69,32 @@ def test_long_rows_many_vectors(cuda, shape, cplx):
         assert np.all(abs(D.to_host(F) - x - got) <= 2.0**-50 * (abs(x) + abs(got)))
         top = ctl[:1].view(torch.float64).item()
         assert abs(top - abs(got).sum(axis=1).max()) <= 1e-12 * top
+
+
+@pytest.mark.parametrize("n,row", [(20000, 24), (5000, 100), (2000, 400), (400, 400)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_single_precision_of_many_vectors(cuda, n, row, cplx):
+    """The root mean square error of an FP32 product of several vectors is no
+    larger than that of one, whose row sums are spread over lanes.  The bound's
+    fifth covers the samples' scatter (a few per cent)."""
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300.sparse import DeviceCSR
+    rng = np.random.default_rng(row)
+    cols = np.sort((np.arange(n)[:, None] + rng.permutation(n)[:row]) % n, axis=1)
+    vals = (rng.normal(size=n * row) + (1j * rng.normal(size=n * row) if cplx else 0.0)).astype(
+        np.complex64 if cplx else np.float32)
+    A = sp.csr_matrix((vals, cols.ravel(), np.arange(n + 1) * row), shape=(n, n))
+    M = DeviceCSR.from_scipy(A)
+    assert M.dtype == vals.dtype
+
+    def error(k):
+        x = (rng.normal(size=(n, k)) + 1j * rng.normal(size=(n, k))).astype(np.complex64)
+        xd = D.to_device(x[:, 0].copy() if k == 1 else x)
+        y = torch.empty_like(xd)
+        M.matvec_into(xd, y)
+        ref = A.astype(np.complex128) @ x.astype(np.complex128)
+        return np.linalg.norm(D.to_host(y).reshape(n, k) - ref) / np.linalg.norm(ref)
+    one = error(1)
+    for k in (2, 3, 5, 8, 13):
+        assert error(k) <= 1.2 * one, k
