@@ -31,8 +31,9 @@
 
 namespace {
 
-// VL: lanes per row group = vectors per sweep of a row; WPL: as vl_row_sum
-template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
+// VL: lanes per row group = vectors per sweep of a row; WPL, LONG: as vl_row_sum
+// (the stacked form's rows are never long: it is not told their number of entries)
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE, bool LONG>
 __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices,
                                         const DV *__restrict__ data, const typename M::BE *__restrict__ Bin,
                                         typename M::BE *__restrict__ Bout, cdbl *__restrict__ F, int64_t nvec,
@@ -89,7 +90,7 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
     }
     __syncthreads();
 
-    const int split = MULTI ? 1 : parts;
+    const int split = LONG ? parts : 1;
     const VlPlace at = vl_place(VL, split);
     const int v = at.v;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -109,7 +110,7 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
             const int64_t c = c0 + v < nvec ? c0 + v : nvec - 1;
             const bool act = valid && at.part == 0 && c0 + v < nvec;
             S ar = M::zero(), ai = M::zero();
-            vl_row_sum<M, DV, true, IT, VMODE, WPL>(indices, data, codes, s_tab, Bin + c,
+            vl_row_sum<M, DV, true, IT, VMODE, WPL, LONG>(indices, data, codes, s_tab, Bin + c,
                                                     (uint32_t)(nvec * sizeof(BE)), at, VL, split, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
@@ -209,25 +210,35 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
         const cdbl *__restrict__ coeff, int j, double tol, void *ctlp
 #define VL_ARGS n, indptr, indices, data, Bin, Bout, F, nvec, VL, split, mu0, mus, sec_off, coeff, j, tol, ctlp
 
-template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE, bool LONG>
 __global__ void __launch_bounds__(256, 3) taylor_vl_kernel(VL_PARAMS)
 {
-    vl_body<M, DV, IT, WPL, MULTI, VMODE>(VL_ARGS);
+    vl_body<M, DV, IT, WPL, MULTI, VMODE, LONG>(VL_ARGS);
 }
 
-template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
-int vl_go(const LpTerm &a)
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE, bool LONG>
+int vl_run(const LpTerm &a, int VL, int split)
 {
     using BE = typename M::BE;
     static int resident = 0;
-    auto k = taylor_vl_kernel<M, DV, IT, WPL, MULTI, VMODE>;
-    const int VL = vl_lanes(a.nvec), split = MULTI ? 1 : vl_split(a.n, a.nnz, VL);
+    auto k = taylor_vl_kernel<M, DV, IT, WPL, MULTI, VMODE, LONG>;
     const int64_t rows = 8 * (32 / (VL * split));       // per block and sweep
     const int blocks = qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident);
     k<<<blocks, 256, 0, a.st>>>(a.n, (const IT *)a.indptr, a.indices, (const DV *)a.data, (const BE *)a.Bin,
                                 (BE *)a.Bout, a.F, a.nvec, VL, split, a.mu0, a.mus, a.sec_off, a.coeff, a.j, a.tol, a.ctl);
     QS_CHECK(cudaGetLastError());
     return QS_OK;
+}
+
+template <class M, class DV, class IT, int WPL, bool MULTI, int VMODE>
+int vl_go(const LpTerm &a)
+{
+    const int VL = vl_lanes(a.nvec);
+    if constexpr (!MULTI) {
+        const int split = vl_split(a.n, a.nnz, VL);
+        if (vl_long<M>(a.n, a.nnz, split)) return vl_run<M, DV, IT, WPL, false, VMODE, true>(a, VL, split);
+    }
+    return vl_run<M, DV, IT, WPL, MULTI, VMODE, false>(a, VL, 1);
 }
 
 template <class M, class DV, class IT, bool MULTI, int VMODE>

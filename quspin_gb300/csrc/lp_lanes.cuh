@@ -89,14 +89,24 @@ static inline int vl_split(int64_t n, int64_t nnz, int VL, int64_t lanes = 10000
 
 constexpr int VB = 4;      // nonzeros of a row in flight
 
-// Chains of a row's sum in one lane, places taken in turn, as the lanes of a row
-// hand-out are chains of their own.  Float pairs take two (four spill: a product of
-// 8 vectors 45.3 -> 47.6 us); plain floats four, summed every VFLUSH batches, since
-// their roundings are what a result is made of: RMS error of a complex64 product
-// of 8 vectors, rows of 24 and 400, 9.3e-8 and 3.6e-7 with two chains, 6.9e-8 and
-// 9.4e-8 so (row hand-out: 6.6e-8 to 9.3e-8 by its lanes, and 1.1e-7).
-template <class M> constexpr int VCHAINS = std::is_same<M, ModeF32>::value ? 4 : 2;
+// Chains of a row's sum in one lane, places taken in turn: two, as two lanes of
+// a row hand-out.  Long rows of plain floats take four, summed every VFLUSH
+// batches, since their roundings are what a result is made of: RMS error of a
+// complex64 product of 8 vectors, rows of 100 and 400 entries, 1.8e-7 and 3.6e-7 with
+// two chains, 8.1e-8 and 9.4e-8 so (row hand-out, 4 and 32 lanes: 1.0e-7 and
+// 1.1e-7).  Four for short rows cost 13% (200 k rows of 20, 32.7 -> 37.1 us), and for
+// float pairs spills (45.3 -> 47.6 us, the L = 20 Ising sector).
+template <class M, bool LONG> constexpr int VCHAINS = LONG && std::is_same<M, ModeF32>::value ? 4 : 2;
 constexpr int VFLUSH = 4;
+
+// Whether an operand takes the kernels for long rows: parts of a row, sweeps in
+// blocks of their own, sums taken now and then.  Their arithmetic costs the others
+// 2 to 5% (a term of 8 vectors, 200 k rows of 20).
+template <class M>
+static inline bool vl_long(int64_t n, int64_t nnz, int split)
+{
+    return split > 1 || (std::is_same<M, ModeF32>::value && n > 0 && nnz / n >= 32);
+}
 
 // A lane's place in its warp: vector v of part `part` of row `grp` of `rows`;
 // lane0: the first lane of its VL.
@@ -116,14 +126,13 @@ __device__ __forceinline__ VlPlace vl_place(int VL, int split)
 // FULL: all of them belong to the row; otherwise only the first `left`.  A
 // word past the row's end is zero and its gather reads column 0: an address
 // without a predicate, its product is skipped.
-template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool FULL, class ST>
+template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool FULL, class ST, int NC>
 __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, const DV *__restrict__ data,
                                          const uint8_t *__restrict__ codes, const DV *tab,
                                          const char *__restrict__ x, ST stride, IT k, int left,
-                                         typename M::S (&ar)[VCHAINS<M>], typename M::S (&ai)[VCHAINS<M>])
+                                         typename M::S (&ar)[NC], typename M::S (&ai)[NC])
 {
     using XE = typename std::conditional<XC, typename M::BE, typename M::S>::type;
-    constexpr int NC = VCHAINS<M>;
     XE xe[VB];
     DV d[VB];
 #pragma unroll
@@ -155,16 +164,19 @@ __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, 
 // the warp fills run without predicates, addresses are one 32 x 32
 // multiply-add, and lanes past the last vector (c clamped by the caller) load
 // and compute like the rest.  Every lane of the warp calls it with its row's
-// range (empty for none).  Parts of a row take every split-th batch of it; the
-// whole sum is in part 0.  x: the vectors' base at vector c; stride: bytes per
-// row of vectors (64 bits where they pass 4 GB).  VMODE: 0 one value per
+// range (empty for none).  LONG: parts of a row take every split-th batch of it,
+// and the whole sum is in part 0.  x: the vectors' base at vector c; stride: bytes
+// per row of vectors (64 bits where they pass 4 GB).  VMODE: 0 one value per
 // nonzero, 1 coded, 2 codes packed into the column words (tab: the 256 values).
-template <class M, class DV, bool XC, class IT, int VMODE, int WPL, class ST>
+template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool LONG, class ST>
 __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, const DV *__restrict__ data,
                                            const uint8_t *__restrict__ codes, const DV *tab, const void *x,
-                                           ST stride, const VlPlace &at, int VL, int split, IT k0, IT k1,
+                                           ST stride, const VlPlace &at, int VL, int parts, IT k0, IT k1,
                                            typename M::S &sr, typename M::S &si)
 {
+    constexpr int NC = VCHAINS<M, LONG>;
+    constexpr bool FLUSH = NC == 4;
+    const int split = LONG ? parts : 1;
     int len = (int)(k1 - k0);
     const int most = __reduce_max_sync(0xffffffffu, len), step = split * VB;
     const int least = __reduce_min_sync(0xffffffffu, at.grp < at.rows ? len : most);   // of the lanes that own a row
@@ -172,8 +184,10 @@ __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, 
     const int v = at.v, lane0 = at.lane0;
     const bool loads = v * WPL < VB;           // the lanes that fetch the words
     // this part's first batch; a lane without a row stays below `least` in a full batch
-    k0 += (IT)(at.part * VB);
-    len -= at.part * VB;
+    if constexpr (LONG) {
+        k0 += (IT)(at.part * VB);
+        len -= at.part * VB;
+    }
     uint32_t word[WPL];
     auto fetch = [&](int b) {
 #pragma unroll
@@ -182,9 +196,9 @@ __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, 
             word[i] = loads && k < len ? (uint32_t)__ldcs(indices + k0 + k) : 0u;
         }
     };
-    typename M::S ar[VCHAINS<M>], ai[VCHAINS<M>];
+    typename M::S ar[NC], ai[NC];
 #pragma unroll
-    for (int i = 0; i < VCHAINS<M>; i++) ar[i] = ai[i] = M::zero();
+    for (int i = 0; i < NC; i++) ar[i] = ai[i] = M::zero();
     fetch(0);
     typename M::S tr = M::zero(), ti = M::zero();
     for (int b = 0, t = 1; b < most; b += step, t++) {
@@ -196,29 +210,30 @@ __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, 
             vl_batch<M, DV, XC, IT, VMODE, WPL, true>(cur, lane0, data, codes, tab, xb, stride, k0 + b, VB, ar, ai);
         else
             vl_batch<M, DV, XC, IT, VMODE, WPL, false>(cur, lane0, data, codes, tab, xb, stride, k0 + b, len - b, ar, ai);
-        if constexpr (VCHAINS<M> == 4) {
+        if constexpr (FLUSH) {
             if (t % VFLUSH == 0) {
                 tr = M::add(tr, M::add(M::add(ar[0], ar[2]), M::add(ar[1], ar[3])));
                 ti = M::add(ti, M::add(M::add(ai[0], ai[2]), M::add(ai[1], ai[3])));
 #pragma unroll
-                for (int i = 0; i < VCHAINS<M>; i++) ar[i] = ai[i] = M::zero();
+                for (int i = 0; i < NC; i++) ar[i] = ai[i] = M::zero();
             }
         }
     }
 #pragma unroll
-    for (int h = VCHAINS<M> / 2; h > 0; h /= 2)
+    for (int h = NC / 2; h > 0; h /= 2)
 #pragma unroll
         for (int i = 0; i < h; i++) {
             ar[i] = M::merge(ar[i], ar[i + h]);
             ai[i] = M::merge(ai[i], ai[i + h]);
         }
-    sr = VCHAINS<M> == 4 ? M::add(tr, ar[0]) : ar[0];
-    si = VCHAINS<M> == 4 ? M::add(ti, ai[0]) : ai[0];
-    for (int o = 1; o < split; o <<= 1) {
-        const int from = (threadIdx.x & 31) + o * VL;
-        sr = M::merge(sr, M::shfl(sr, from));
-        si = M::merge(si, M::shfl(si, from));
-    }
+    sr = FLUSH ? M::add(tr, ar[0]) : ar[0];
+    si = FLUSH ? M::add(ti, ai[0]) : ai[0];
+    if constexpr (LONG)
+        for (int o = 1; o < split; o <<= 1) {
+            const int from = (threadIdx.x & 31) + o * VL;
+            sr = M::merge(sr, M::shfl(sr, from));
+            si = M::merge(si, M::shfl(si, from));
+        }
 }
 
 }  // namespace

@@ -230,11 +230,12 @@ __global__ void __launch_bounds__(256) spmv_lz_kernel(LzProduct p, int lgG)
 // 194 us then, 120 us now; 5 vectors 112 / 87 us; J1-J2 L = 28 (361 k rows,
 // 10.7 M real nonzeros): 8 vectors 401 / 191 us, 2 vectors 98 / 69 us.  Complex
 // pairs run at three blocks per SM (four spill: 129 us), the rest at four.
-template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST>
+// LONG: as vl_row_sum, with sweeps of the vectors for gridDim.y.
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST, bool LONG>
 __global__ void __launch_bounds__(256, std::is_same<DV, cpf>::value ? 3 : 4)
 spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restrict__ indices,
                const DV *__restrict__ data, const void *__restrict__ xv, YT *__restrict__ y, int64_t nvec, int VL,
-               int split, cdbl a, int overwrite, const unsigned long long *__restrict__ xnorm)
+               int parts, cdbl a, int overwrite, const unsigned long long *__restrict__ xnorm)
 {
     using S = typename M::S;
     using XE = typename std::conditional<XC, typename M::BE, S>::type;
@@ -254,6 +255,8 @@ spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restri
     __syncthreads();
     const cx<S> av{s_a[0], s_a[1]};
     const int k2 = s_k;
+    const int split = LONG ? parts : 1;
+    const int64_t first = LONG ? (int64_t)blockIdx.y * VL : 0, sweep = LONG ? (int64_t)gridDim.y * VL : VL;
     const VlPlace at = vl_place(VL, split);
     const int v = at.v;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -262,13 +265,13 @@ spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restri
         const int64_t r = rb + at.grp;
         const bool valid = r < n && at.grp < at.rows;
         const IT k0 = valid ? indptr[r] : (IT)0, k1 = valid ? indptr[r + 1] : (IT)0;
-        // all sweeps, or one of them for each gridDim.y
-        for (int64_t c0 = (int64_t)blockIdx.y * VL; c0 < nvec; c0 += (int64_t)gridDim.y * VL) {
+        for (int64_t c0 = first; c0 < nvec; c0 += sweep) {
             const int64_t c = c0 + v < nvec ? c0 + v : nvec - 1;
             const bool act = valid && at.part == 0 && c0 + v < nvec;
             S ar = M::zero(), ai = M::zero();
-            vl_row_sum<M, DV, XC, IT, VM, WPL>(indices, data, codes, s_tab, reinterpret_cast<const XE *>(xv) + c,
-                                               (ST)(nvec * sizeof(XE)), at, VL, split, k0, k1, ar, ai);
+            vl_row_sum<M, DV, XC, IT, VM, WPL, LONG>(indices, data, codes, s_tab,
+                                                     reinterpret_cast<const XE *>(xv) + c, (ST)(nvec * sizeof(XE)),
+                                                     at, VL, split, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
                 const S accr = M::fin(ar);
@@ -364,17 +367,14 @@ int spmv_go(const SpmvArgs &a)
     return QS_OK;
 }
 
-template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST = uint32_t>
-int spmm_go(const SpmvArgs &a)
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST, bool LONG>
+int spmm_run(const SpmvArgs &a, int VL, int split, int64_t lanes)
 {
     static int resident = 0;
-    auto k = spmm_vl_kernel<M, DV, XC, YT, IT, VM, WPL, ST>;
-    // FP32 arithmetic leaves more of the latency to hide than float pairs do
-    const int64_t lanes = std::is_same<M, ModeF32>::value ? 130000 : 100000;
-    const int VL = vl_lanes(a.nvec), split = vl_split(a.n, a.nnz, VL, lanes);
+    auto k = spmm_vl_kernel<M, DV, XC, YT, IT, VM, WPL, ST, LONG>;
     const int64_t rows = 8 * (32 / (VL * split));       // per block and sweep
     // with few rows the sweeps go to blocks of their own, too
-    int64_t apart = lanes / (a.n * VL * split);
+    int64_t apart = LONG ? lanes / (a.n * VL * split) : 1;
     if (apart > 65535) apart = 65535;
     if (apart > (a.nvec + VL - 1) / VL) apart = (a.nvec + VL - 1) / VL;
     const dim3 grid(qs_persistent_grid(k, 256, (a.n + rows - 1) / rows, resident), (unsigned)(apart < 1 ? 1 : apart));
@@ -382,6 +382,18 @@ int spmm_go(const SpmvArgs &a)
                               split, a.a, a.overwrite, a.xnorm);
     QS_CHECK(cudaGetLastError());
     return QS_OK;
+}
+
+template <class M, class DV, bool XC, class YT, class IT, int VM, int WPL, class ST = uint32_t>
+int spmm_go(const SpmvArgs &a)
+{
+    // FP32 arithmetic leaves more of the latency to hide than float pairs do
+    const int64_t lanes = std::is_same<M, ModeF32>::value ? 130000 : 100000;
+    const int VL = vl_lanes(a.nvec), split = vl_split(a.n, a.nnz, VL, lanes);
+    if constexpr (sizeof(ST) == 4) {
+        if (!vl_long<M>(a.n, a.nnz, split)) return spmm_run<M, DV, XC, YT, IT, VM, WPL, ST, false>(a, VL, 1, lanes);
+    }
+    return spmm_run<M, DV, XC, YT, IT, VM, WPL, ST, true>(a, VL, split, lanes);
 }
 
 template <class M, class DV, bool XC, class YT, class IT, int VM>
