@@ -111,7 +111,7 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
             const bool act = valid && at.part == 0 && c0 + v < nvec;
             S ar = M::zero(), ai = M::zero();
             vl_row_sum<M, DV, true, IT, VMODE, WPL, LONG>(indices, data, codes, s_tab, Bin + c,
-                                                    (uint32_t)(nvec * sizeof(BE)), at, VL, split, k0, k1, ar, ai);
+                                                    (uint32_t)(nvec * sizeof(BE)), v, at.lane0, at.part, at.grp < at.rows, VL, split, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
                 const BE bo = M::ldB(Bin + e);

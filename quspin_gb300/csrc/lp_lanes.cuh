@@ -171,7 +171,7 @@ __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, 
 template <class M, class DV, bool XC, class IT, int VMODE, int WPL, bool LONG, class ST>
 __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, const DV *__restrict__ data,
                                            const uint8_t *__restrict__ codes, const DV *tab, const void *x,
-                                           ST stride, const VlPlace &at, int VL, int parts, IT k0, IT k1,
+                                           ST stride, int v, int lane0, int part, bool owns, int VL, int parts, IT k0, IT k1,
                                            typename M::S &sr, typename M::S &si)
 {
     constexpr int NC = VCHAINS<M, LONG>;
@@ -179,14 +179,13 @@ __device__ __forceinline__ void vl_row_sum(const int32_t *__restrict__ indices, 
     const int split = LONG ? parts : 1;
     int len = (int)(k1 - k0);
     const int most = __reduce_max_sync(0xffffffffu, len), step = split * VB;
-    const int least = __reduce_min_sync(0xffffffffu, at.grp < at.rows ? len : most);   // of the lanes that own a row
+    const int least = __reduce_min_sync(0xffffffffu, owns ? len : most);   // of the lanes that own a row
     const char *xb = reinterpret_cast<const char *>(x);
-    const int v = at.v, lane0 = at.lane0;
     const bool loads = v * WPL < VB;           // the lanes that fetch the words
     // this part's first batch; a lane without a row stays below `least` in a full batch
     if constexpr (LONG) {
-        k0 += (IT)(at.part * VB);
-        len -= at.part * VB;
+        k0 += (IT)(part * VB);
+        len -= part * VB;
     }
     uint32_t word[WPL];
     auto fetch = [&](int b) {

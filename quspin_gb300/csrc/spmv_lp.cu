@@ -257,7 +257,17 @@ spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restri
     const int k2 = s_k;
     const int split = LONG ? parts : 1;
     const int64_t first = LONG ? (int64_t)blockIdx.y * VL : 0, sweep = LONG ? (int64_t)gridDim.y * VL : VL;
-    const VlPlace at = vl_place(VL, split);
+    // the short form written out: with vl_place the compiler's schedule of the whole
+    // loop is up to 5% slower (70 k rows of 24, 8 vectors, 41.3 against 39.4 us)
+    VlPlace at;
+    if constexpr (LONG) at = vl_place(VL, split);
+    else {
+        at.rows = 32 / VL;
+        at.grp = (threadIdx.x & 31) / VL;
+        at.lane0 = at.grp * VL;
+        at.v = (threadIdx.x & 31) - at.lane0;
+        at.part = 0;
+    }
     const int v = at.v;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -271,7 +281,7 @@ spmm_vl_kernel(int64_t n, const IT *__restrict__ indptr, const int32_t *__restri
             S ar = M::zero(), ai = M::zero();
             vl_row_sum<M, DV, XC, IT, VM, WPL, LONG>(indices, data, codes, s_tab,
                                                      reinterpret_cast<const XE *>(xv) + c, (ST)(nvec * sizeof(XE)),
-                                                     at, VL, split, k0, k1, ar, ai);
+                                                     v, at.lane0, at.part, at.grp < at.rows, VL, split, k0, k1, ar, ai);
             if (act) {
                 const int64_t e = r * nvec + c;
                 const S accr = M::fin(ar);
