@@ -460,7 +460,7 @@ struct EnumArgs {
 // out, so a chunk's representatives are found in its own order.
 // Measured at L = 28, Sz = 0, k = 0, p = z = +1 (40.1 M candidates, 112
 // elements): 4.76 ms a pass with full checks in step and byte tables, 0.82 ms so
-// (issue slots 67% busy).
+// (issue slots 60% busy, the integer pipe as much).
 //
 // Queues, map tables and binomials share the block's dynamic memory; what
 // does not fit there (a dozen maps from byte tables at 64 sites) gives way
@@ -1029,7 +1029,7 @@ __device__ __forceinline__ int64_t term_element(const SymView<S> &V, const Basis
 // works.  Slices of the terms keep the chip filled on small sectors.
 // Measured at L = 28 (358 k kets, 112 hopping terms, 112 elements): a count or
 // fill pass 6.9 ms with one search per thread and term, 0.95 ms so (integer
-// pipe 74% busy); the matrix-free apply at L = 26 2.22 ms before, 0.29 ms now.
+// pipe 77% busy); the matrix-free apply at L = 26 2.22 ms before, 0.29 ms now.
 // The queues lie before the map tables in the block's dynamic memory; where
 // both do not fit, the block has fewer warps (elem_launch).
 #define ELEM_WARPS 4

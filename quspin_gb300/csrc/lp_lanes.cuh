@@ -159,8 +159,8 @@ __device__ __forceinline__ void vl_batch(const uint32_t (&cur)[WPL], int lane0, 
 // the VL vectors' entries of a nonzero as one contiguous piece.  The group's
 // column words are loaded VB at a time, WPL per lane (one, or two where VL is 2
 // or 3), a batch ahead of their use, and handed round by shuffles.  The loop is
-// bound by its instruction count (issue slots 73% busy in the product with 8
-// vectors), nearly all of it float-pair arithmetic: batches that every row of
+// bound by its instruction count (issue slots 64% busy in the product of the L = 20
+// Ising sector with 8 vectors), nearly all of it float-pair arithmetic: batches that every row of
 // the warp fills run without predicates, addresses are one 32 x 32
 // multiply-add, and lanes past the last vector (c clamped by the caller) load
 // and compute like the rest.  Every lane of the warp calls it with its row's

@@ -22,6 +22,10 @@
 // L = 32, where the term vectors, F and the words exceed L2 together: 1.98 -> 1.04
 // GB, 1.02 times what the padded words and the vectors once come to.
 //
+// The layout is of the sliced ELLPACK family (A. Monakov, A. Lokhmotov and A.
+// Avetisyan, HiPEAC 2010; SELL-C-sigma, M. Kreutzer et al., SIAM J. Sci. Comput. 36
+// (2014) C401-C423); the order of a slice's nonzeros over its slots is this file's.
+//
 // Words: col << 8 | code as in the packed form, PAD where a row has no nonzero
 // in the slot; slots in groups of four, a group as 32 x 16 bytes, so that a
 // lane loads four of its words at once.  sptr[s]: groups before slice s.

@@ -124,8 +124,8 @@ class DeviceCSR:
     def _spmv_operand(self, products=1):
         """The float-pair operand of the next ``products`` products: plain pairs for the
         first CODE_AFTER_PRODUCTS products of a matrix, then the coded form
-        (one sort of the values, worth it for a reused matrix; at once when
-        a Taylor operand exists), with the codes packed into the column words
+        (two or three streaming passes over the values, csrc/codes.cu, worth
+        it for a reused matrix; at once when a Taylor operand exists), with the codes packed into the column words
         where that applies."""
         P = self.__dict__.get("_paired_coded")
         if P is None:
