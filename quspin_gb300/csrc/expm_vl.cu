@@ -91,7 +91,17 @@ __device__ __forceinline__ void vl_body(int64_t n, const IT *__restrict__ indptr
     __syncthreads();
 
     const int split = LONG ? parts : 1;
-    const VlPlace at = vl_place(VL, split);
+    // the short form written out: with vl_place the compiler's schedule of the whole
+    // loop is up to 18% slower (a complex64 term of 8 vectors, 1.3 M rows of 27)
+    VlPlace at;
+    if constexpr (LONG) at = vl_place(VL, split);
+    else {
+        at.rows = 32 / VL;
+        at.grp = (threadIdx.x & 31) / VL;
+        at.lane0 = at.grp * VL;
+        at.v = (threadIdx.x & 31) - at.lane0;
+        at.part = 0;
+    }
     const int v = at.v;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
