@@ -115,3 +115,26 @@ def test_reorth_adaptive_second_pass_when_norm_lost(cuda, cplx):
     np.testing.assert_array_equal(out, two)
     assert np.abs(Qh.conj() @ out).max() <= 1e-12 * np.linalg.norm(out)
     np.testing.assert_allclose(out, 1e-6 * q[:, nk], rtol=0, atol=1e-15)
+
+
+@pytest.mark.parametrize("nk", [1, 15, 16, 17, 33, 64])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_projection_row_counts(cuda, nk, cplx):
+    """One Gram-Schmidt pass over row counts around the sixteen that a lane has
+    in flight.  Tolerance: sums of nk and of n products in FP64."""
+    import torch
+    from quspin_gb300 import _device as D
+    from quspin_gb300 import _lib
+    rng = np.random.default_rng(nk)
+    n = 3001
+    Q = rng.normal(size=(nk, n)) + (1j * rng.normal(size=(nk, n)) if cplx else 0.0)
+    Q /= np.linalg.norm(Q, axis=1, keepdims=True)
+    r = rng.normal(size=n) + (1j * rng.normal(size=n) if cplx else 0.0)
+    Qd, rd = D.to_device(Q), D.to_device(r)
+    L = _lib.load()
+    scr = D.scratch_doubles(L.qs_lanczos_reorth_scratch_doubles(nk))
+    ctl = torch.zeros(2, dtype=torch.int32, device="cuda")
+    _lib.call("qs_lanczos_reorth", n, int(cplx), nk, D.ptr(Qd), n, D.ptr(rd), 1, D.ptr(scr), D.ptr(ctl), D.stream())
+    h = Q.conj() @ r
+    bound = 1e-15 * (nk + 60) * (abs(Q).T @ (abs(Q) @ abs(r)) + abs(r))
+    assert np.all(abs(D.to_host(rd) - (r - Q.T @ h)) <= bound)
